@@ -252,7 +252,8 @@ int mt_plan_create(const mt_grid_desc* desc, mt_plan** out) {
 int mt_plan_destroy(mt_plan* p) {
   if (!p) return MT_OK;
   void* ptrs[] = {p->d_lstart, p->d_theta, p->d_gauss, p->d_plm, p->d_dplm, p->d_dlh,
-                  p->d_wq,     p->d_wq_v,  p->d_ost2,  p->d_cosn, p->d_twiddle};
+                  p->d_wq,     p->d_wq_v,  p->d_ost2,  p->d_cosn, p->d_twiddle,
+                  p->d_phi_tw1};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   free_split_tables(p);
@@ -1368,7 +1369,7 @@ static int nl_anel_split_t(const mt_plan* p, int n_r, const mt_anel_in* in,
 // The digit-split anelastic stage runs where one CTA of its FP64 phi stage
 // holds a (theta row, level)'s buffers in shared memory.
 static bool anel_ozaki_fits(const mt_plan* p, int mag, int chem) {
-  return nl_anel_f64_smem(p->n_phi, mag, chem) > 0;
+  return nl_anel_f64_smem(p->tab, mag, chem) > 0;
 }
 
 // Fused anelastic stage in digit-split precision: the synthesis row programs

@@ -19,6 +19,7 @@ OUT = os.path.join(PKG, "libmagic_b200.so")
 BUILD = os.path.join(ROOT, "_build")
 
 SOURCES = ["api.cu", "tables.cu", "legendre_f64.cu", "fourier.cu", "nonlinear.cu",
+           "nl_bouss_f64.cu", "nl_bouss_oz.cu", "nl_anel_f64.cu",
            "split_tables.cu", "legendre_split.cu", "nl_split.cu", "split_transforms.cu",
            "nl_anel_split.cu", "radial_td.cu",
            "implicit.cu", "energy.cu", "ozaki.cu", "batch.cu"]
@@ -59,7 +60,7 @@ def build(verbose=False, force=False):
         if all(os.path.getmtime(s) <= t for s in srcs + hdrs + [os.path.abspath(__file__)]):
             return OUT
     os.makedirs(BUILD, exist_ok=True)
-    with cf.ThreadPoolExecutor(max_workers=min(8, len(SOURCES))) as ex:
+    with cf.ThreadPoolExecutor(max_workers=min(os.cpu_count() or 8, len(SOURCES))) as ex:
         res = list(ex.map(lambda s: _compile(s, verbose), SOURCES))
     if verbose:
         for _, log in res:

@@ -50,6 +50,8 @@ struct Tables {
   const double* ost2;      // (n_theta) interleaved rows: 1/sin^2
   const double* cosn;      // (n_theta) interleaved rows: cos/sin^2
   const double2* twiddle;  // (n_phi) exp(-2 pi i n / n_phi)
+  const double2* phi_tw1;  // twiddles of the outer step of the row FFTs (phi_fft.cuh)
+  int fft_a, fft_b, fft_f; // n_phi / 2 = fft_a fft_b fft_f (phi_fft.cuh)
   int fft_nstages;
   int fft_radix[kMaxFftStages];
 };
@@ -72,6 +74,7 @@ struct mt_plan {
   double* d_ost2 = nullptr;
   double* d_cosn = nullptr;
   double2* d_twiddle = nullptr;
+  double2* d_phi_tw1 = nullptr;
   mt::Tables tab;              // device pointers + sizes, ready for launches
   // split-precision operand planes (null in FP64 plans)
   void* split = nullptr;

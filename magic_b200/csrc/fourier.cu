@@ -2,132 +2,183 @@
 //
 // Every grid row is one real field: synthesis is irfft(norm="forward")
 // (unnormalised, Im of mode 0 ignored), analysis rfft(norm="forward"), both
-// through a half-length complex FFT (fft.cuh).  Analysis outputs are scaled
-// by 1/N and by the row's quadrature weight (2 pi w, or 2 pi w/sin^2 for
-// vector components), so the Legendre analysis needs only P and dP.
-#include "fft.cuh"
+// through a half-length complex FFT in shared memory (phi_fft.cuh).  Analysis
+// outputs are scaled by 1/N and by the row's quadrature weight (2 pi w, or
+// 2 pi w/sin^2 for vector components), so the Legendre analysis needs only P
+// and dP.
 #include "fourier.cuh"
+#include "phi_fft.cuh"
 
 namespace mt {
 
 constexpr int kColsPerCta = 8;  // real columns (grid rows) per CTA
 constexpr int kFftThreads = 256;
 
-// Expand the half spectra staged at row[0..M) (zero above) into Z (in place).
-template <typename R>
-__device__ __forceinline__ void c2r_prepare(cplx<R>* row, int H, const double2* __restrict__ tw,
-                                            int tid, int nthr) {
-  for (int k = tid; k <= H / 2; k += nthr) {
-    int kc = H - k;
-    cplx<R> Xk = row[pad16(k)];
-    if (k == 0) {
-      Xk.y = 0;  // irfft ignores Im X[0]; X[H] is zero (2 (n_m - 1) < N)
-      row[pad16(0)] = c2r_pre(Xk, cplx<R>{0, 0}, 0, tw);
-    } else {
-      cplx<R> Xc = row[pad16(kc)];
-      cplx<R> Zk = c2r_pre(Xk, Xc, k, tw);
-      cplx<R> Zc = c2r_pre(Xc, Xk, kc, tw);
-      row[pad16(k)] = Zk;
-      if (kc != k) row[pad16(kc)] = Zc;
+template <class SH>
+__global__ void __launch_bounds__(kFftThreads, SH::kMax <= 12 ? 3 : 2)
+    k_fourier_to_grid(ToGridArgs a) {
+  extern __shared__ double smem[];
+  cplx<double>* buf = reinterpret_cast<cplx<double>*>(smem);
+  const Tables& t = a.t;
+  const SH sh(t);
+  const int H = sh.H, N = 2 * H, M = t.n_m, nt = t.n_theta;
+  const int row = blockIdx.y;
+  const int col0 = blockIdx.x * kColsPerCta;
+  const int ncol = min(kColsPerCta, a.ncols - col0);
+  cplx<double>* tw1 = buf + kColsPerCta * sh.S;
+  cplx<double>* twN = tw1 + (sh.A - 1) * sh.Ns;
+  phi_twiddles_to_smem(tw1, sh, t);
+  const double2* Fr = a.F + (int64_t)row * a.f_row + col0;
+  const float rcp = 1.0f / (float)ncol;
+  // pairs (k, H - k) of every column: Z[k] = c2r_pre(X[k], X[H - k]) with X = 0
+  // at k >= M (and X[H] = 0: 2 (n_m - 1) < N), kLd pairs in flight per thread
+  constexpr int kLd = 4;
+  const int total = (H / 2 + 1) * ncol;
+  for (int e0 = 0; e0 < total; e0 += kLd * kFftThreads) {
+    double2 xa[kLd], xb[kLd];
+#pragma unroll
+    for (int u = 0; u < kLd; ++u) {
+      const int e = e0 + u * kFftThreads + threadIdx.x, k = fdiv(e, rcp), q = e - k * ncol;
+      xa[u] = xb[u] = make_double2(0.0, 0.0);
+      if (e < total) {
+        if (k < M) xa[u] = __ldg(&Fr[k * a.f_m + q]);
+        if (k > 0 && H - k < M) xb[u] = __ldg(&Fr[(H - k) * a.f_m + q]);
+      }
+    }
+    if (e0 == 0) {  // the tables are complete once every thread's copies are
+      cp_async_wait_all();
+      __syncthreads();
+    }
+#pragma unroll
+    for (int u = 0; u < kLd; ++u) {
+      const int e = e0 + u * kFftThreads + threadIdx.x, k = fdiv(e, rcp), q = e - k * ncol;
+      if (e < total) {
+        cplx<double>* z = buf + q * sh.S;
+        const cplx<double> w = twN[k];
+        const cplx<double> Xk = {xa[u].x, k ? xa[u].y : 0.0}, Xc = {xb[u].x, xb[u].y};
+        z[phi_slot(sh, k)] = c2r_pre_d(Xk, Xc, w);
+        if (k > 0 && 2 * k < H)  // exp(-2 pi i (H - k) / N) = -conj(w)
+          z[phi_slot(sh, H - k)] = c2r_pre_d(Xc, Xk, cplx<double>{-w.x, w.y});
+      }
+    }
+  }
+  __syncthreads();
+  phi_inverse(buf, ncol, sh, tw1);
+  // one warp per row; lanes take consecutive complex points n = p + A s < A B
+  const int lane = threadIdx.x & 31, AB = sh.A * sh.B;
+  for (int q = threadIdx.x >> 5; q < ncol; q += kFftThreads / 32) {
+    const int c = col0 + q, f = c / a.B, b = c - f * a.B;
+    double* dst = a.out[f] + ((int64_t)b * nt + row) * N;
+    const bool wide = (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
+    auto put = [&](int n, double x, double y) {
+      if (wide) reinterpret_cast<double2*>(dst)[n] = make_double2(x, y);
+      else {
+        dst[2 * n] = x;
+        dst[2 * n + 1] = y;
+      }
+    };
+    for (int n = lane; n < AB; n += 32) {
+      const int s = sh.divA(n), p = n - s * sh.A;
+      const cplx<double>* z = buf + q * sh.S + p * sh.P + s;
+      const cplx<double> x = z[0];
+      if (sh.F == 2) {
+        const cplx<double> y = z[sh.B];
+        put(n, x.x + y.x, x.y + y.y);
+        put(n + AB, x.x - y.x, x.y - y.y);
+      } else {
+        put(n, x.x, x.y);
+      }
     }
   }
 }
 
-__global__ void __launch_bounds__(kFftThreads) k_fourier_to_grid(ToGridArgs a) {
+template <class SH>
+__global__ void __launch_bounds__(kFftThreads, SH::kMax <= 12 ? 3 : 2)
+    k_grid_to_fourier(ToFourierArgs a) {
   extern __shared__ double smem[];
   cplx<double>* buf = reinterpret_cast<cplx<double>*>(smem);
   const Tables& t = a.t;
-  const int N = t.n_phi, H = N / 2, M = t.n_m, nt = t.n_theta;
-  const int stride = padded_len(H);
+  const SH sh(t);
+  const int H = sh.H, N = 2 * H, M = t.n_m, nt = t.n_theta;
   const int row = blockIdx.y;
   const int col0 = blockIdx.x * kColsPerCta;
   const int ncol = min(kColsPerCta, a.ncols - col0);
-  cplx<double>* tws = buf + (kColsPerCta + kFftRowBatch) * stride;
-  fft_twiddles_to_smem(tws, H, t.twiddle, t.fft_radix, t.fft_nstages);
-  for (int i = threadIdx.x; i < ncol * stride; i += blockDim.x) buf[i] = {0.0, 0.0};
-  __syncthreads();
-  const double2* Fr = a.F + (int64_t)row * a.f_row + col0;
-  const float rcp = 1.0f / (float)ncol;
-  for (int e = threadIdx.x; e < M * ncol; e += blockDim.x) {
-    int k = fdiv(e, rcp), q = e - k * ncol;
-    cp_async16(&buf[q * stride + pad16(k)], &Fr[k * a.f_m + q]);
+  cplx<double>* tw1 = buf + kColsPerCta * sh.S;
+  cplx<double>* twN = tw1 + (sh.A - 1) * sh.Ns;
+  phi_twiddles_to_smem(tw1, sh, t);
+  const int lane = threadIdx.x & 31, AB = sh.A * sh.B;
+  for (int q = threadIdx.x >> 5; q < ncol; q += kFftThreads / 32) {
+    const int c = col0 + q, f = c / a.B, b = c - f * a.B;
+    const double2* src =
+        reinterpret_cast<const double2*>(a.in[f] + ((int64_t)b * nt + row) * N);
+#pragma unroll 4
+    for (int n = lane; n < AB; n += 32) {
+      const int s = sh.divA(n), p = n - s * sh.A;
+      cplx<double>* z = buf + q * sh.S + p * sh.P + s;
+      const double2 x = __ldg(&src[n]);
+      if (sh.F == 2) {
+        const double2 y = __ldg(&src[n + AB]);
+        z[0] = {x.x + y.x, x.y + y.y};
+        z[sh.B] = {x.x - y.x, x.y - y.y};
+      } else {
+        z[0] = {x.x, x.y};
+      }
+    }
   }
   cp_async_wait_all();
   __syncthreads();
-  for (int q = threadIdx.x / 64; q < ncol; q += kFftThreads / 64)
-    c2r_prepare(buf + q * stride, H, t.twiddle, threadIdx.x % 64, 64);
-  __syncthreads();
-  fft_rows<true>(buf, buf + kColsPerCta * stride, ncol, H, stride, t.fft_radix, t.fft_nstages, tws);
-  const float rcpN = 1.0f / (float)N;
-  for (int e = threadIdx.x; e < ncol * N; e += blockDim.x) {
-    int q = fdiv(e, rcpN), n = e - q * N;
-    cplx<double> z = buf[q * stride + pad16(n >> 1)];
-    int c = col0 + q;
-    int f = c / a.B, b = c % a.B;
-    a.out[f][((int64_t)b * nt + row) * N + n] = (n & 1) ? z.y : z.x;
-  }
-}
-
-__global__ void __launch_bounds__(kFftThreads) k_grid_to_fourier(ToFourierArgs a) {
-  extern __shared__ double smem[];
-  cplx<double>* buf = reinterpret_cast<cplx<double>*>(smem);
-  const Tables& t = a.t;
-  const int N = t.n_phi, H = N / 2, M = t.n_m, nt = t.n_theta;
-  const int stride = padded_len(H);
-  const int row = blockIdx.y;
-  const int col0 = blockIdx.x * kColsPerCta;
-  const int ncol = min(kColsPerCta, a.ncols - col0);
-  cplx<double>* tws = buf + (kColsPerCta + kFftRowBatch) * stride;
-  fft_twiddles_to_smem(tws, H, t.twiddle, t.fft_radix, t.fft_nstages);
-  const float rcpH = 1.0f / (float)H;
-  for (int e = threadIdx.x; e < ncol * H; e += blockDim.x) {
-    int q = fdiv(e, rcpH), h = e - q * H;
-    int c = col0 + q;
-    const double* src = a.in[c / a.B] + ((int64_t)(c % a.B) * nt + row) * N;
-    double2 v = *reinterpret_cast<const double2*>(src + 2 * h);
-    buf[q * stride + pad16(h)] = {v.x, v.y};
-  }
-  __syncthreads();
-  fft_rows<false>(buf, buf + kColsPerCta * stride, ncol, H, stride, t.fft_radix, t.fft_nstages, tws);
+  phi_forward(buf, ncol, sh, tw1);
   const double w = (a.vector ? t.wq_v[row] : t.wq[row]) / N;
   double2* Fr = a.F + (int64_t)row * a.f_row + col0;
   const float rcpc = 1.0f / (float)ncol;
-  for (int e = threadIdx.x; e < M * ncol; e += blockDim.x) {
-    int k = fdiv(e, rcpc), q = e - k * ncol;
-    const cplx<double>* z = buf + q * stride;
-    cplx<double> X = r2c_post(z[pad16(k)], z[pad16((H - k) % H)], k, t.twiddle);
+#pragma unroll 4
+  for (int e = threadIdx.x; e < M * ncol; e += kFftThreads) {
+    const int k = fdiv(e, rcpc), q = e - k * ncol;
+    const cplx<double>* z = buf + q * sh.S;
+    const cplx<double> X = r2c_post_d(z[phi_slot(sh, k)], z[phi_slot(sh, k ? H - k : 0)], twN[k]);
     Fr[k * a.f_m + q] = make_double2(w * X.x, w * X.y);
   }
 }
 
 static size_t fft_smem(const Tables& t) {
-  return ((size_t)(kColsPerCta + kFftRowBatch) * padded_len(t.n_phi / 2) + t.n_phi / 2) *
-         sizeof(double2);
+  return ((size_t)kColsPerCta * phi_row_len(t) + phi_tw_len(t)) * sizeof(double2);
+}
+
+template <int kMax>
+static int launch_to_grid(const ToGridArgs& a, cudaStream_t st) {
+  const size_t sm = fft_smem(a.t);
+  auto kern = k_fourier_to_grid<PhiShapeRt<kMax>>;
+  MT_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  dim3 grid((a.ncols + kColsPerCta - 1) / kColsPerCta, a.t.n_theta);
+  kern<<<grid, kFftThreads, sm, st>>>(a);
+  MT_CHECK_CUDA(cudaGetLastError());
+  return MT_OK;
+}
+
+template <int kMax>
+static int launch_to_fourier(const ToFourierArgs& a, cudaStream_t st) {
+  const size_t sm = fft_smem(a.t);
+  auto kern = k_grid_to_fourier<PhiShapeRt<kMax>>;
+  MT_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  dim3 grid((a.ncols + kColsPerCta - 1) / kColsPerCta, a.t.n_theta);
+  kern<<<grid, kFftThreads, sm, st>>>(a);
+  MT_CHECK_CUDA(cudaGetLastError());
+  return MT_OK;
 }
 
 int launch_fourier_to_grid(const ToGridArgs& a, cudaStream_t st) {
-  size_t sm = fft_smem(a.t);
-  MT_CHECK_CUDA(cudaFuncSetAttribute(k_fourier_to_grid, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)sm));
-  dim3 grid((a.ncols + kColsPerCta - 1) / kColsPerCta, a.t.n_theta);
-  k_fourier_to_grid<<<grid, kFftThreads, sm, st>>>(a);
-  MT_CHECK_CUDA(cudaGetLastError());
-  return MT_OK;
+  const int r = phi_max_radix(a.t);
+  if (r <= 12) return launch_to_grid<12>(a, st);
+  return r <= 18 ? launch_to_grid<18>(a, st) : launch_to_grid<27>(a, st);
 }
 
 int launch_grid_to_fourier(const ToFourierArgs& a, cudaStream_t st) {
-  size_t sm = fft_smem(a.t);
-  MT_CHECK_CUDA(cudaFuncSetAttribute(k_grid_to_fourier, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)sm));
-  dim3 grid((a.ncols + kColsPerCta - 1) / kColsPerCta, a.t.n_theta);
-  k_grid_to_fourier<<<grid, kFftThreads, sm, st>>>(a);
-  MT_CHECK_CUDA(cudaGetLastError());
-  return MT_OK;
+  const int r = phi_max_radix(a.t);
+  if (r <= 12) return launch_to_fourier<12>(a, st);
+  return r <= 18 ? launch_to_fourier<18>(a, st) : launch_to_fourier<27>(a, st);
 }
 
-// Largest n_phi the fused stage's shared memory holds: 14 field rows plus a
-// 7-row scratch of H = n_phi/2 padded complex FP64 values and the H-point
-// twiddle table within 227 KB.
+// Largest n_phi that the row FFTs' two radices cover (phi_fft.cuh).
 int fft_max_nphi() { return 1168; }
 
 }  // namespace mt

@@ -56,6 +56,8 @@ struct NlBoussArgs {
 };
 
 int launch_nl_bouss(bool mag, bool chem, const NlBoussArgs& a, cudaStream_t st);
+int launch_nl_bouss_f64(bool mag, bool chem, const NlBoussArgs& a, cudaStream_t st);
+int launch_nl_bouss_oz(bool mag, bool chem, const NlBoussArgs& a, cudaStream_t st);
 int launch_courant_finish(int n_r, const unsigned long long* vr2, const unsigned long long* vh2,
                           const double* delxr2, const double* delxh2, double* dtr, double* dth,
                           cudaStream_t st);

@@ -105,7 +105,7 @@ int launch_nl_anel_split(bool mag, bool chem, const NlAnelArgs& a, cudaStream_t 
 // FP64 anelastic phi stage; its dynamic shared memory (0 where n_phi is too
 // long for one CTA's buffers)
 int launch_nl_anel_f64(bool mag, bool chem, const NlAnelArgs& a, cudaStream_t st);
-size_t nl_anel_f64_smem(int n_phi, bool mag, bool chem);
+size_t nl_anel_f64_smem(const Tables& t, bool mag, bool chem);
 
 // phi stage of the split drop-in transforms (split_transforms.cu); rows are
 // (column b, field f), r = b * nf + f

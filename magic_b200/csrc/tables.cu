@@ -137,6 +137,41 @@ static int factor_radices(int n, int* out) {
   return n == 1 ? ns : -1;
 }
 
+// tw[(q - 1) Ns + slot] = exp(-2 pi i q j / H), 1 <= q < A, slot < Ns = F B of
+// wavenumber j = F (slot % B) + slot / B (phi_fft.cuh).
+__global__ void k_phi_tw1(int A, int B, int F, double2* tw) {
+  const int Ns = F * B, i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= (A - 1) * Ns) return;
+  const int q = i / Ns + 1, slot = i % Ns, j = F * (slot % B) + slot / B;
+  double s, c;
+  sincospi(2.0 * (q * j) / (A * Ns), &s, &c);
+  tw[i] = make_double2(c, -s);
+}
+
+// H = a b f of the row FFTs: f = 2 for even H; among the pairs of supported
+// radices the lowest register class of the kernels (radices up to 12, 18, 27)
+// first, then an outer radix a that is a multiple of 8 (no bank conflicts in
+// the inner step), then the smallest larger radix; false if H has a factor other
+// than 2, 3, 5.
+static bool phi_factor(int H, int* a, int* b, int* f) {
+  static const int radix[] = {1, 2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16, 18, 20, 25, 27};
+  *f = H % 2 == 0 ? 2 : 1;
+  const int n = H / *f;
+  int best = 1 << 30;
+  for (int x : radix)
+    for (int y : radix) {
+      if (x * y != n) continue;
+      const int m = x > y ? x : y, cls = m <= 12 ? 0 : m <= 18 ? 1 : 2;
+      const int score = cls * 10000 + (x % 8 ? 1000 : 0) + 10 * m + (x < y);
+      if (score < best) {
+        best = score;
+        *a = x;
+        *b = y;
+      }
+    }
+  return best < 1 << 30;
+}
+
 int build_tables(mt_plan* p) {
   const int nt = p->n_theta, nhs = p->nhs;
   std::vector<int> ls(p->n_m);
@@ -149,7 +184,9 @@ int build_tables(mt_plan* p) {
   int radix[kMaxFftStages];
   MT_REQUIRE(p->n_phi % 2 == 0, MT_ERR_UNSUPPORTED, "n_phi_max must be even");
   int nst = factor_radices(p->n_phi / 2, radix);  // real FFTs run as half-length complex FFTs
-  MT_REQUIRE(nst > 0, MT_ERR_UNSUPPORTED, "n_phi_max must factor into 2, 3, 5");
+  int fa = 1, fb = 1, ff = 1;
+  MT_REQUIRE(nst > 0 && phi_factor(p->n_phi / 2, &fa, &fb, &ff), MT_ERR_UNSUPPORTED,
+             "n_phi_max must factor into 2, 3, 5");
 
   size_t tsz = (size_t)p->lm_max * nhs * sizeof(double);
   MT_CHECK_CUDA(cudaMalloc(&p->d_lstart, p->n_m * sizeof(int)));
@@ -163,6 +200,8 @@ int build_tables(mt_plan* p) {
   MT_CHECK_CUDA(cudaMalloc(&p->d_ost2, nt * sizeof(double)));
   MT_CHECK_CUDA(cudaMalloc(&p->d_cosn, nt * sizeof(double)));
   MT_CHECK_CUDA(cudaMalloc(&p->d_twiddle, p->n_phi * sizeof(double2)));
+  const int n_tw1 = (fa - 1) * ff * fb;
+  MT_CHECK_CUDA(cudaMalloc(&p->d_phi_tw1, (n_tw1 + 1) * sizeof(double2)));
   MT_CHECK_CUDA(cudaMemcpy(p->d_lstart, ls.data(), p->n_m * sizeof(int), cudaMemcpyHostToDevice));
 
   k_gauleg<<<(nt / 2 + 127) / 128, 128>>>(nt, p->d_theta, p->d_gauss);
@@ -173,6 +212,7 @@ int build_tables(mt_plan* p) {
                                    p->d_cosn);
   k_lm<<<(p->lm_max + 255) / 256, 256>>>(p->l_max, p->minc, p->lm_max, p->d_dlh);
   k_twiddle<<<(p->n_phi + 255) / 256, 256>>>(p->n_phi, p->d_twiddle);
+  k_phi_tw1<<<n_tw1 / 256 + 1, 256>>>(fa, fb, ff, p->d_phi_tw1);
   MT_CHECK_CUDA(cudaGetLastError());
   MT_CHECK_CUDA(cudaDeviceSynchronize());
 
@@ -193,6 +233,10 @@ int build_tables(mt_plan* p) {
   t.ost2 = p->d_ost2;
   t.cosn = p->d_cosn;
   t.twiddle = p->d_twiddle;
+  t.phi_tw1 = p->d_phi_tw1;
+  t.fft_a = fa;
+  t.fft_b = fb;
+  t.fft_f = ff;
   t.fft_nstages = nst;
   for (int s = 0; s < kMaxFftStages; ++s) t.fft_radix[s] = s < nst ? radix[s] : 1;
   return MT_OK;
