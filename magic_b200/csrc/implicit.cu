@@ -683,6 +683,195 @@ __global__ void __launch_bounds__(Bounds<kStaged, kNt == 2 ? 3 : 2>::kThreads,
   }
 }
 
+// ---------------------------------------------------------------------------
+// Dense operators (Chebyshev levels): the solve and the radial derivatives both
+// on the FP64 tensor pipe, as one chain of contractions over the CTA's 16
+// orders (32 real rows, the A operand in shared memory): x = rhs M_l^T, then
+// D x with the transposed derivative matrices as B.  All operators stream
+// through one ring of three buffers (cp.async, two chunks in flight, one
+// barrier per chunk), the derivatives' first chunks while the solve finishes.
+// Warp w owns the n-tiles (8 output levels) w, w + nwarps, ... for every m-tile
+// and keeps all of its accumulators in registers to the epilogue, where lanes
+// of the two parts of an order swap halves so that each holds one complex
+// level: the stores are 128 contiguous bytes per order.
+// FP64 FMAs run at 24 TFLOP/s on this part, the tensor pipe at 37; the FMA form
+// re-read D1 and D2 from L2 once per four orders.  The anelastic implicit
+// updates at l_max 383, n_r 129 (S, Z, (w, p)): 6.09 -> 4.73 ms; the Boussinesq
+// ones at l_max 127, n_r 65: 389 -> 319 us, at l_max 64, n_r 33: 124 -> 100 us.
+// Tensor pipe 52 % busy (field) and 43 % ((w, p), one CTA per SM by registers).
+constexpr int kDnMaxTiles = 9;  // warps per CTA
+
+// rows of B: chunk rows [0, nrow) from src (row stride ld, even), zeros from
+// row nvalid on, into dst
+__device__ __forceinline__ void dn_stage(const double* src, int nvalid, int nrow, int ld,
+                                         double* dst) {
+  const int nv = nrow * ld / 2, lim = nvalid * ld / 2;
+  for (int i = threadIdx.x; i < nv; i += blockDim.x) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst + 2 * i);
+    const int n = i < lim ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d),
+                 "l"(i < lim ? src + 2 * i : src), "r"(n)
+                 : "memory");
+  }
+}
+
+// acc[i][t] += A(m-tile t, rows k0 ..) B(n-tile warp + i nwarps) over KC rows of
+// a staged chunk; A element of m-tile t at k: order 4 t + ar / 2, part ar % 2.
+template <int kNt, int KC>
+__device__ __forceinline__ void dn_mma(const double* fd, int a_off, int fs, int K, int k0,
+                                       const double* mb, int ld, int nt_n, int tmax,
+                                       double (&acc)[kNt][4][2]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  const int ar = lane >> 2, ac = lane & 3;
+#pragma unroll
+  for (int q = 0; q < KC / 4; ++q) {
+    const int kk = 4 * q + ac, k = k0 + kk;
+    double av[4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+      av[t] = (t < tmax && k < K) ? fd[a_off + (4 * t * fs + k) * 2] : 0.0;
+#pragma unroll
+    for (int i = 0; i < kNt; ++i) {
+      const int nt = warp + i * nwarp;
+      if (nt < nt_n) {
+        const double bv = mb[kk * ld + 8 * nt + ar];
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+          if (t < tmax) dmma_f64(acc[i][t], av[t], bv);
+      }
+    }
+  }
+}
+
+// The lane's complex value of an accumulator pair: lanes of part 0 get level
+// 8 nt + 2 ac, lanes of part 1 (four lanes up) level 8 nt + 2 ac + 1.
+__device__ __forceinline__ double2 dn_pair(const double (&c)[2]) {
+  const int p = (threadIdx.x >> 2) & 1;
+  const double got = __shfl_xor_sync(0xffffffffu, p ? c[0] : c[1], 4);
+  return p ? double2{got, c[1]} : double2{c[0], got};
+}
+
+template <int kNt>
+__device__ __forceinline__ void dn_zero(double (&acc)[kNt][4][2]) {
+#pragma unroll
+  for (int i = 0; i < kNt; ++i)
+#pragma unroll
+    for (int t = 0; t < 4; ++t) acc[i][t][0] = acc[i][t][1] = 0.0;
+}
+
+// accumulators of the solve over the right-hand sides in f (imaginary part of
+// m = 0 dropped)
+template <int kNt>
+__device__ __forceinline__ void dn_store_x(double* fd, int fs, int n, int nt_n, int mc0,
+                                           const double (&acc)[kNt][4][2]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  const int ar = lane >> 2, ac = lane & 3;
+#pragma unroll
+  for (int i = 0; i < kNt; ++i) {
+    const int nt = warp + i * nwarp;
+    if (nt >= nt_n) continue;
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const int o = 4 * t + (ar >> 1), p = ar & 1;
+      const bool drop = p && mc0 + o == 0;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int j = 8 * nt + 2 * ac + h;
+        if (j < n) fd[(o * fs + j) * 2 + p] = drop ? 0.0 : acc[i][t][h];
+      }
+    }
+  }
+}
+
+// Registers: the accumulators of both derivatives (16 kNt doubles) stay live.
+template <int kNt>
+__global__ void __launch_bounds__(32 * kDnMaxTiles, kNt == 1 ? 3 : kNt == 2 ? 2 : 1)
+    k_update_field_dense(UsArgs a) {
+  extern __shared__ __align__(16) double2 dnbuf[];
+  __shared__ int lm_row[4 * kRows];
+  constexpr int rows = 4 * kRows;
+  const int n_r = a.n_r, ldm = a.ldm, fs = a.fs, l = blockIdx.y, mc0 = blockIdx.x * rows;
+  const int nrow = cta_rows(mc0, rows, l, a.minc, a.n_m);
+  if (nrow == 0) return;
+  double2* f = dnbuf;                           // [rows][fs]: rhs, then x
+  double* fd = reinterpret_cast<double*>(f);
+  double* ring = (double*)(dnbuf + rows * fs);  // 3 x [kKc][ldm]
+  const double* Ml = a.mt + (int64_t)l * n_r * ldm;
+  // chunks: nS of kKc rows of M_l, then nD of kKc / 2 rows each of D1 and D2
+  constexpr int KD = kKc / 2;
+  const int nS = (n_r + kKc - 1) / kKc, nD = (n_r + KD - 1) / KD;
+  auto stage = [&](int c) {
+    double* b = ring + (c % 3) * kKc * ldm;
+    if (c < nS) {
+      dn_stage(Ml + (int64_t)c * kKc * ldm, min(kKc, n_r - c * kKc), kKc, ldm, b);
+    } else if (c < nS + nD) {
+      const int k0 = (c - nS) * KD, nv = min(KD, n_r - k0);
+      dn_stage(a.D1.dense + (int64_t)k0 * ldm, nv, KD, ldm, b);
+      dn_stage(a.D2.dense + (int64_t)k0 * ldm, nv, KD, ldm, b + KD * ldm);
+    }
+    cpa_commit();
+  };
+  stage(0);
+  stage(1);
+  if (threadIdx.x < rows)
+    lm_row[threadIdx.x] = threadIdx.x < nrow
+        ? a.lstart[mc0 + threadIdx.x] + (l - (mc0 + threadIdx.x) * a.minc) : 0;
+  __syncthreads();
+  build_rhs<false, 3>(a, l, rows, nrow, lm_row, f);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  const int ar = lane >> 2, ac = lane & 3, nt_n = (n_r + 7) >> 3;
+  const int a_off = (ar >> 1) * fs * 2 + (ar & 1), tmax = (nrow + kRows - 1) / kRows;
+  int c = 0;
+  {
+    double acc[kNt][4][2];
+    dn_zero(acc);
+    for (; c < nS; ++c) {
+      cpa_wait<1>();
+      __syncthreads();
+      stage(c + 2);
+      dn_mma<kNt, kKc>(fd, a_off, fs, n_r, c * kKc, ring + (c % 3) * kKc * ldm, ldm, nt_n, tmax,
+                       acc);
+    }
+    __syncthreads();
+    dn_store_x(fd, fs, n_r, nt_n, mc0, acc);
+  }
+  double d1[kNt][4][2], d2[kNt][4][2];
+  dn_zero(d1);
+  dn_zero(d2);
+  for (; c < nS + nD; ++c) {
+    cpa_wait<1>();
+    __syncthreads();
+    stage(c + 2);
+    const double* b = ring + (c % 3) * kKc * ldm;
+    const int k0 = (c - nS) * KD;
+    dn_mma<kNt, KD>(fd, a_off, fs, n_r, k0, b, ldm, nt_n, tmax, d1);
+    dn_mma<kNt, KD>(fd, a_off, fs, n_r, k0, b + KD * ldm, ldm, nt_n, tmax, d2);
+  }
+  const double so_l = a.so_l ? a.so_l[l] : 1.0, ia_l = a.ia_l[l], ic_l = a.ic_l[l];
+#pragma unroll
+  for (int i = 0; i < kNt; ++i) {
+    const int nt = warp + i * nwarp;
+    if (nt >= nt_n) continue;
+    const int j = 8 * nt + 2 * ac + (ar & 1), jc = min(j, n_r - 1);
+    const double so = so_l * (a.so_r ? a.so_r[jc] : 1.0);
+    const double c1 = a.ib_r[jc], c0 = (a.ic_r ? a.ic_r[jc] : 0.0) + ic_l * a.ic_r2[jc];
+    const double ia = ia_l * a.ia_r[jc];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const double2 x1 = dn_pair(d1[i][t]), x2 = dn_pair(d2[i][t]);
+      const int row = 4 * t + (ar >> 1);
+      if (row >= nrow || j >= n_r) continue;
+      const int64_t o = (int64_t)lm_row[row] * a.ld + j;
+      const double2 v = f[row * fs + j];
+      a.x[o] = v;
+      a.dx[o] = x1;
+      if (a.d2x) a.d2x[o] = x2;
+      a.old[o] = double2{so * v.x, so * v.y};
+      a.impl[o] = double2{ia * (x2.x + c1 * x1.x - c0 * v.x), ia * (x2.y + c1 * x1.y - c0 * v.y)};
+    }
+  }
+}
+
 struct PwArgs {
   int n_r, ldm, fs, l_max, minc, n_m, groups;
   BandView band;
@@ -857,7 +1046,7 @@ constexpr int kWpRows = 8;
 constexpr int kWpThreads = 256;
 
 struct WpArgs {
-  int n_r, ldm, l_max, minc, n_m;
+  int n_r, ldm, ldd, l_max, minc, n_m;  // ldd: row stride of the dense derivatives
   const int* lstart;
   double2 *w, *dw, *ddw, *p, *dp, *wo, *wi, *we0, *we1, *po, *pi, *pe0, *pe1;
   const double2 *s, *xi;
@@ -1022,25 +1211,18 @@ __global__ void __launch_bounds__(kWpThreads) k_update_wp(WpArgs a) {
   }
 }
 
-// The same update with the coupled solve on the FP64 tensor pipe, for
-// 2 n_r <= 64 kNt (kNt n-tiles of 8 levels per warp): CTA = 16 orders (4
-// m-tiles) of one degree, 8 warps.  The rows' right-hand sides (w part, then p
-// part, row stride fs) are the A operand of solve_tile_dmma with the
-// 2 n_r x 2 n_r operator streamed through shared memory in 16-row chunks; the
-// solution overwrites them.  Derivatives: thread = (4-row group, level), each
-// D coefficient serving 4 rows.  kNt = 4 with 8 warps covers 2 n_r <= 256
-// (two CTAs per SM by registers); kNt = 6 with 9 warps covers 2 n_r <= 432 and
-// runs up to n_r = 192 (e.g. the 129 Chebyshev levels of the anelastic
-// benchmark; its shared memory allows one CTA per SM anyway).
-// The six-tile variant runs 9 warps: 129 levels give 33 n-tiles (at most four
-// per warp) and 4 x 129 derivative items (two rounds of 288 threads, where 256
-// threads would need a third round for four items).
-constexpr int kWpDmmaMaxR = 128;
+// The same update with the coupled solve on the FP64 tensor pipe, for 144 < n_r
+// <= 192 (or operators that are not dense): CTA = 16 orders (4 m-tiles) of one
+// degree, 9 warps, at most kNt = 6 n-tiles of 8 levels per warp.  The rows'
+// right-hand sides (w part, then p part, row stride fs) are the A operand of
+// solve_tile_dmma with the 2 n_r x 2 n_r operator streamed through shared
+// memory in 16-row chunks; the solution overwrites them.  Derivatives: thread =
+// (4-row group, level), each D coefficient serving 4 rows.
 constexpr int kWpDmmaWideMaxR = 192;
-__host__ __device__ constexpr int wp_dmma_threads(int kNt) { return kNt == 4 ? 256 : 288; }
+constexpr int kWpDmmaThreads = 288;
 
 template <int kNt>
-__global__ void __launch_bounds__(wp_dmma_threads(kNt), kNt == 4 ? 2 : 1)
+__global__ void __launch_bounds__(kWpDmmaThreads, 1)
     k_update_wp_dmma(WpArgs a, int fs) {
   extern __shared__ __align__(16) double2 wpd[];
   __shared__ int lm_row[4 * kRows];
@@ -1096,6 +1278,165 @@ __global__ void __launch_bounds__(wp_dmma_threads(kNt), kNt == 4 ? 2 : 1)
       if (row >= nrow) break;
       wp_store(a, c, (int64_t)lm_row[row] * a.ld + j, xw[r * fs + j], xw[r * fs + n_r + j],
                d1[r], d2[r], d3[r], dp[r]);
+    }
+  }
+}
+
+// The same update with everything on the FP64 tensor pipe (dense D1, D2, D3; see
+// k_update_field_dense), for 2 n_r <= 72 kNt: the coupled solve, then D1 w and
+// D1 p in one pass over D1, then D2 w and D3 w.  After the first pass the parts
+// of both implicit terms that need w, p, D1 w and D1 p are folded into two
+// values per level, so that no more than two sets of derivative accumulators
+// are live.  The nine warps of one CTA per SM (kNt = 4) hold every accumulator
+// in registers.
+template <int kNt>
+__global__ void __launch_bounds__(32 * kDnMaxTiles, kNt == 2 ? 2 : 1)
+    k_update_wp_dense(WpArgs a, int fs, int ring_len) {
+  constexpr int kNd = kNt / 2, rows = 4 * kRows;  // n-tiles per warp: solve, derivatives
+  extern __shared__ __align__(16) double2 wpn[];
+  __shared__ int lm_row[rows];
+  const int n_r = a.n_r, n2 = 2 * n_r, l = blockIdx.y, mc0 = blockIdx.x * rows;
+  const int nrow = cta_rows(mc0, rows, l, a.minc, a.n_m);
+  if (nrow == 0) return;
+  double2* f = wpn;                               // [rows][fs]: (w, p) right-hand sides, then w, p
+  double* fd = reinterpret_cast<double*>(f);
+  double* ring = (double*)(wpn + rows * fs);      // 3 x ring_len
+  const int ldm = a.ldm, ldd = a.ldd;
+  const double* Ml = a.mt + (int64_t)l * n2 * ldm;
+  // chunks of kKc rows: nS of M_l, nD of D1, nD of (D2, D3)
+  const int nS = l > 0 ? (n2 + kKc - 1) / kKc : 0, nD = (n_r + kKc - 1) / kKc;
+  auto stage = [&](int c) {
+    double* b = ring + (c % 3) * ring_len;
+    if (c < nS) {
+      dn_stage(Ml + (int64_t)c * kKc * ldm, min(kKc, n2 - c * kKc), kKc, ldm, b);
+    } else if (c < nS + 2 * nD) {
+      const bool second = c >= nS + nD;
+      const int k0 = (c - nS - (second ? nD : 0)) * kKc, nv = min(kKc, n_r - k0);
+      dn_stage((second ? a.D2.dense : a.D1.dense) + (int64_t)k0 * ldd, nv, kKc, ldd, b);
+      if (second) dn_stage(a.D3.dense + (int64_t)k0 * ldd, nv, kKc, ldd, b + kKc * ldd);
+    }
+    cpa_commit();
+  };
+  stage(0);
+  stage(1);
+  if (threadIdx.x < rows)
+    lm_row[threadIdx.x] = threadIdx.x < nrow
+        ? a.lstart[mc0 + threadIdx.x] + (l - (mc0 + threadIdx.x) * a.minc) : 0;
+  __syncthreads();
+  const double2 zero = {0.0, 0.0};
+#pragma unroll 2
+  for (int e = threadIdx.x; e < rows * n_r; e += blockDim.x) {
+    const int r = e / n_r, k = e - r * n_r;
+    double2 vw = zero, vp = zero;
+    if (r < nrow) wp_rhs(a, (int64_t)lm_row[r] * a.ld + k, k, vw, vp);
+    f[r * fs + k] = vw;
+    f[r * fs + n_r + k] = vp;
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  const int ar = lane >> 2, ac = lane & 3, nt_s = (n2 + 7) >> 3, nt_d = (n_r + 7) >> 3;
+  const int a_off = (ar >> 1) * fs * 2 + (ar & 1), tmax = (nrow + kRows - 1) / kRows;
+  int c = 0;
+  if (l == 0) {
+    // degree 0, one row: w = 0, the l = 0 pressure from its own right-hand side
+    // (built in the row's p half, then solved into the w half and copied)
+    __syncthreads();
+    const int64_t row0 = (int64_t)lm_row[0] * a.ld;
+    for (int k = threadIdx.x; k < n_r; k += blockDim.x)
+      f[n_r + k] = double2{wp_p0_rhs(a, row0, k), 0.0};
+    __syncthreads();
+    for (int j = threadIdx.x; j < n_r; j += blockDim.x)
+      f[j] = double2{op_row(a.P0, f + n_r, j).x, 0.0};
+    __syncthreads();
+    for (int j = threadIdx.x; j < n_r; j += blockDim.x) {
+      f[n_r + j] = f[j];
+      f[j] = zero;
+    }
+  } else {
+    double acc[kNt][4][2];
+    dn_zero(acc);
+    for (; c < nS; ++c) {
+      cpa_wait<1>();
+      __syncthreads();
+      stage(c + 2);
+      dn_mma<kNt, kKc>(fd, a_off, fs, n2, c * kKc, ring + (c % 3) * ring_len, ldm, nt_s, tmax,
+                       acc);
+    }
+    __syncthreads();
+    dn_store_x(fd, fs, n2, nt_s, mc0, acc);
+  }
+  double2 tw[kNd][4], tp[kNd][4];
+  {
+    double d1[kNd][4][2], dp[kNd][4][2];
+    dn_zero(d1);
+    dn_zero(dp);
+    for (; c < nS + nD; ++c) {
+      cpa_wait<1>();
+      __syncthreads();
+      stage(c + 2);
+      const double* b = ring + (c % 3) * ring_len;
+      const int k0 = (c - nS) * kKc;
+      dn_mma<kNd, kKc>(fd, a_off, fs, n_r, k0, b, ldd, nt_d, tmax, d1);
+      dn_mma<kNd, kKc>(fd + 2 * n_r, a_off, fs, n_r, k0, b, ldd, nt_d, tmax, dp);
+    }
+#pragma unroll
+    for (int i = 0; i < kNd; ++i) {
+      const int nt = warp + i * nwarp;
+      if (nt >= nt_d) continue;
+      const int j = 8 * nt + 2 * ac + (ar & 1);
+      const WpCoef q = wp_coef(a, l, min(j, n_r - 1));
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const double2 x1 = dn_pair(d1[i][t]), xp = dn_pair(dp[i][t]);
+        const int row = 4 * t + (ar >> 1);
+        tw[i][t] = tp[i][t] = zero;
+        if (row >= nrow || j >= n_r) continue;
+        const int64_t o = (int64_t)lm_row[row] * a.ld + j;
+        const double2 w = f[row * fs + j], p = f[row * fs + n_r + j];
+        const double2 sv = a.s[o], xv = a.xi ? a.xi[o] : zero;
+        a.w[o] = w;
+        a.dw[o] = x1;
+        a.p[o] = p;
+        a.dp[o] = xp;
+        a.wo[o] = double2{q.dLo * w.x, q.dLo * w.y};
+        a.po[o] = double2{-q.dLo * x1.x, -q.dLo * x1.y};
+        tw[i][t].x = -xp.x + q.beta * p.x + q.fw * (q.cw1 * x1.x - q.cw0 * w.x) +
+                     q.rg * (a.BuoFac * sv.x + a.ChemFac * xv.x);
+        tw[i][t].y = -xp.y + q.beta * p.y + q.fw * (q.cw1 * x1.y - q.cw0 * w.y) +
+                     q.rg * (a.BuoFac * sv.y + a.ChemFac * xv.y);
+        tp[i][t].x = q.dLo * p.x + q.fw * (q.cp1 * x1.x - q.cp0 * w.x);
+        tp[i][t].y = q.dLo * p.y + q.fw * (q.cp1 * x1.y - q.cp0 * w.y);
+      }
+    }
+  }
+  double d2[kNd][4][2], d3[kNd][4][2];
+  dn_zero(d2);
+  dn_zero(d3);
+  for (; c < nS + 2 * nD; ++c) {
+    cpa_wait<1>();
+    __syncthreads();
+    stage(c + 2);
+    const double* b = ring + (c % 3) * ring_len;
+    const int k0 = (c - nS - nD) * kKc;
+    dn_mma<kNd, kKc>(fd, a_off, fs, n_r, k0, b, ldd, nt_d, tmax, d2);
+    dn_mma<kNd, kKc>(fd, a_off, fs, n_r, k0, b + kKc * ldd, ldd, nt_d, tmax, d3);
+  }
+#pragma unroll
+  for (int i = 0; i < kNd; ++i) {
+    const int nt = warp + i * nwarp;
+    if (nt >= nt_d) continue;
+    const int j = 8 * nt + 2 * ac + (ar & 1);
+    const WpCoef q = wp_coef(a, l, min(j, n_r - 1));
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const double2 x2 = dn_pair(d2[i][t]), x3 = dn_pair(d3[i][t]);
+      const int row = 4 * t + (ar >> 1);
+      if (row >= nrow || j >= n_r) continue;
+      const int64_t o = (int64_t)lm_row[row] * a.ld + j;
+      a.ddw[o] = x2;
+      const bool z = q.zero_impl;
+      a.wi[o] = z ? zero : double2{tw[i][t].x + q.fw * x2.x, tw[i][t].y + q.fw * x2.y};
+      a.pi[o] = z ? zero : double2{tp[i][t].x + q.fw * (q.cp2 * x2.x - x3.x),
+                                   tp[i][t].y + q.fw * (q.cp2 * x2.y - x3.y)};
     }
   }
 }
@@ -1211,11 +1552,7 @@ int mt_lop_create(int n_l, int n_r, const double* M, mt_lop** out) {
              "bad per-degree operator argument");
   *out = nullptr;
   const size_t per = (size_t)n_r * n_r;
-  // j stride: a multiple of 8 (the tensor-pipe n-tiles read whole 8-level
-  // groups), 8 (mod 16) so that the 4 k rows of a B fragment fall on distinct
-  // bank halves
-  int ldm = (n_r + 7) / 8 * 8;
-  if (ldm % 16 == 0) ldm += 8;
+  const int ldm = lop_ld(n_r);
   const size_t per_t = (size_t)n_r * ldm;
   std::vector<double> t(per_t * n_l, 0.0);
   for (int l = 0; l < n_l; ++l)
@@ -1401,6 +1738,20 @@ int mt_update_field(const mt_plan* p, int n_r, const mt_field_update* u, const m
   a.band = BandView{solve->abd, solve->piv, solve->fr, solve->fc, solve->kl, solve->ku, nullptr};
   a.D1 = radial_op_view(D1);
   a.D2 = radial_op_view(D2);
+  if (!solve->abd && n_r <= kStagedMaxR && D1->dense && D2->dense) {
+    const int nt_n = (n_r + 7) / 8, tiles = (nt_n + kDnMaxTiles - 1) / kDnMaxTiles;
+    a.fs = n_r + ((4 - n_r) & 7);  // conflict-free A fragments
+    const size_t sm = (size_t)4 * kRows * a.fs * sizeof(double2) +
+                      (size_t)3 * kKc * a.ldm * sizeof(double);
+    auto kern = tiles == 1   ? k_update_field_dense<1>
+                : tiles == 2 ? k_update_field_dense<2>
+                             : k_update_field_dense<4>;
+    MT_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    const dim3 grid((p->n_m + 4 * kRows - 1) / (4 * kRows), p->l_max + 1);
+    kern<<<grid, 32 * ((nt_n + tiles - 1) / tiles), sm, (cudaStream_t)stream>>>(a);
+    MT_CHECK_CUDA(cudaGetLastError());
+    return MT_OK;
+  }
   const TileLaunch t = tile_launch(n_r, a.ldm, p->l_max, p->n_m, 1,
                                    solve->abd ? band_smem_bytes(solve->kl, solve->ku, n_r) : 0);
   MT_REQUIRE(!t.staged || (n_r + 7) / 8 <= t.nt * (t.threads / 32), MT_ERR_ARG,
@@ -1558,17 +1909,29 @@ int mt_update_wp(const mt_plan* p, int n_r, const mt_wp_update* u, const mt_lop*
   a.D2 = radial_op_view(D2);
   a.D3 = radial_op_view(D3);
   a.P0 = radial_op_view(P0);
+  const int nt_s = (2 * n_r + 7) / 8, tiles = (nt_s + kDnMaxTiles - 1) / kDnMaxTiles;
+  if (tiles <= 4 && D1->dense && D2->dense && D3->dense) {  // n_r <= 144
+    const int fs = 2 * n_r + ((4 - 2 * n_r) & 7);
+    a.ldd = lop_ld(n_r);
+    const int ring = kKc * std::max(a.ldm, 2 * a.ldd);
+    const size_t sm = (size_t)4 * kRows * fs * sizeof(double2) + (size_t)3 * ring * sizeof(double);
+    auto kern = tiles <= 2 ? k_update_wp_dense<2> : k_update_wp_dense<4>;
+    MT_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    const dim3 grid((p->n_m + 4 * kRows - 1) / (4 * kRows), p->l_max + 1);
+    kern<<<grid, 32 * ((nt_s + tiles - 1) / tiles), sm, (cudaStream_t)stream>>>(a, fs, ring);
+    MT_CHECK_CUDA(cudaGetLastError());
+    return MT_OK;
+  }
   if (n_r <= kWpDmmaWideMaxR) {
     // tensor-pipe tiling: rows 4 (mod 8) double2 apart (conflict-free A
     // fragments), the operator's 16-row chunks double-buffered
     const int fs = 2 * n_r + ((4 - 2 * n_r) & 7);
     const size_t sm = (size_t)4 * kRows * fs * sizeof(double2) +
                       (size_t)2 * kKc * a.ldm * sizeof(double);
-    const bool narrow = n_r <= kWpDmmaMaxR;
-    auto kern = narrow ? k_update_wp_dmma<4> : k_update_wp_dmma<6>;
+    auto kern = k_update_wp_dmma<6>;
     MT_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     const dim3 grid((p->n_m + 4 * kRows - 1) / (4 * kRows), p->l_max + 1);
-    kern<<<grid, wp_dmma_threads(narrow ? 4 : 6), sm, (cudaStream_t)stream>>>(a, fs);
+    kern<<<grid, kWpDmmaThreads, sm, (cudaStream_t)stream>>>(a, fs);
     MT_CHECK_CUDA(cudaGetLastError());
     return MT_OK;
   }

@@ -8,14 +8,26 @@ struct mt_radial_op {
   int n_r = 0, W = 0, device = 0;
   int* k0 = nullptr;       // (n_r) first column of each row's band
   double* vals = nullptr;  // (W, n_r) band-transposed values: vals[kk * n_r + j] = D[j][k0[j] + kk]
+  double* dense = nullptr; // W = n_r: D transposed, (n_r, lop_ld(n_r)), zero past n_r (else null)
 };
 
 namespace mt {
+
+// Row stride of the transposed operators that the tensor-pipe tiles read (solve
+// operators, dense derivatives): a multiple of 8 (the n-tiles read whole 8-level
+// groups), 8 (mod 16) so that the 4 k rows of a B fragment fall on distinct bank
+// halves.
+constexpr int kDenseMaxR = 256;  // largest n_r with a transposed dense copy
+inline int lop_ld(int n) {
+  const int ld = (n + 7) / 8 * 8;
+  return ld % 16 == 0 ? ld + 8 : ld;
+}
 
 struct OpView {
   int n_r, W;
   const int* k0;
   const double* vals;
+  const double* dense;
 };
 
 // (D f)[j] for one complex row f staged in shared memory
@@ -32,7 +44,7 @@ __device__ __forceinline__ double2 op_row(const OpView& op, const double2* f, in
 }
 
 inline OpView radial_op_view(const mt_radial_op* op) {
-  return OpView{op->n_r, op->W, op->k0, op->vals};
+  return OpView{op->n_r, op->W, op->k0, op->vals, op->dense};
 }
 inline int radial_op_size(const mt_radial_op* op) { return op ? op->n_r : 0; }
 // non-null and built on the current device (radial_td.cu)

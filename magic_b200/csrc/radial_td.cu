@@ -276,6 +276,7 @@ int mt_radial_op_create(int n_r, const double* D, mt_radial_op** out) {
   auto fail = [&](int rc) {
     if (op->k0) cudaFree(op->k0);
     if (op->vals) cudaFree(op->vals);
+    if (op->dense) cudaFree(op->dense);
     delete op;
     return rc;
   };
@@ -286,6 +287,16 @@ int mt_radial_op_create(int n_r, const double* D, mt_radial_op** out) {
       cudaMemcpy(op->vals, vals.data(), vals.size() * sizeof(double), cudaMemcpyHostToDevice) !=
           cudaSuccess)
     return fail((set_error("radial operator allocation or upload failed"), MT_ERR_CUDA));
+  if (W == n_r && n_r <= kDenseMaxR) {
+    const int ld = lop_ld(n_r);
+    std::vector<double> t((size_t)n_r * ld, 0.0);
+    for (int k = 0; k < n_r; ++k)
+      for (int j = 0; j < n_r; ++j) t[(size_t)k * ld + j] = D[(size_t)j * n_r + k];
+    if (cudaMalloc(&op->dense, t.size() * sizeof(double)) != cudaSuccess ||
+        cudaMemcpy(op->dense, t.data(), t.size() * sizeof(double), cudaMemcpyHostToDevice) !=
+            cudaSuccess)
+      return fail((set_error("radial operator allocation or upload failed"), MT_ERR_CUDA));
+  }
   *out = op;
   return MT_OK;
 }
@@ -311,6 +322,7 @@ int mt_radial_op_destroy(mt_radial_op* op) {
   if (!op) return MT_OK;
   if (op->k0) cudaFree(op->k0);
   if (op->vals) cudaFree(op->vals);
+  if (op->dense) cudaFree(op->dense);
   delete op;
   return MT_OK;
 }
