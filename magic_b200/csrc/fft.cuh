@@ -1,4 +1,6 @@
-// Shared-memory FFTs of the phi stage.
+// Shared-memory FFTs of the phi stage: complex arithmetic, register DFTs, and the
+// block-wide Stockham chain of the FP32 Boussinesq stage at row lengths without
+// a half-warp form (the other kernels use phi_fft.cuh and fft_hw.cuh).
 //
 // Each real field row of length N = n_phi is transformed on its own through a
 // complex FFT of half length H = N/2 (z_n = x_2n + i x_2n+1), so rounding of
@@ -202,20 +204,18 @@ __device__ __forceinline__ void fft_stage(const cplx<R>* __restrict__ src, cplx<
   __syncthreads();
 }
 
-constexpr int kFftRowBatch = 7;  // rows per pass through the scratch buffer
-
 // Full transform of `nrows` rows (in place), ping-ponging each batch of at
-// most kFftRowBatch rows through `scratch` (kFftRowBatch * stride values).
+// most `batch` rows through `scratch` (batch * stride values).
 // Radices come from the plan (product H, each of 2, 3, 4, 5, 8); tw holds the
 // stages' twiddle tables one after another (fft_twiddles_to_smem, H - 1 values).
 template <bool INV, typename R>
-__device__ __forceinline__ void fft_rows(cplx<R>* buf, cplx<R>* scratch, int nrows, int H,
-                                         int stride, const int* radix, int nstages,
+__device__ __forceinline__ void fft_rows(cplx<R>* buf, cplx<R>* scratch, int nrows, int batch,
+                                         int H, int stride, const int* radix, int nstages,
                                          const cplx<R>* __restrict__ tw) {
-  for (int r0 = 0; r0 < nrows; r0 += kFftRowBatch) {
+  for (int r0 = 0; r0 < nrows; r0 += batch) {
     cplx<R>* a = buf + r0 * stride;
     cplx<R>* b = scratch;
-    const int nr = min(kFftRowBatch, nrows - r0);
+    const int nr = min(batch, nrows - r0);
     int Ns = 1, off = 0;
     for (int s = 0; s < nstages; ++s) {
       int rad = radix[s];
@@ -305,6 +305,23 @@ __device__ __forceinline__ cplx<R> r2c_post(cplx<R> Zk, cplx<R> Zc, int k,
   cplx<R> e = {(R)w.x, (R)w.y};  // exp(-2 pi i k/N)
   cplx<R> t = cmul(D, e);
   // X = F - (i/2) e D  with the factor 1/2 on both terms
+  return {(R)0.5 * (F.x + t.y), (R)0.5 * (F.y - t.x)};
+}
+
+// The same with the twiddle wN = exp(-2 pi i k / N) at hand.
+template <typename R>
+__device__ __forceinline__ cplx<R> c2r_pre(cplx<R> Xk, cplx<R> Xc, cplx<R> wN) {
+  const cplx<R> cXc = conj(Xc);
+  const cplx<R> F = cadd(Xk, cXc), D = csub(Xk, cXc);
+  const cplx<R> G = cmul(D, conj(wN));
+  return {F.x - G.y, F.y + G.x};  // F + i G
+}
+
+template <typename R>
+__device__ __forceinline__ cplx<R> r2c_post(cplx<R> Zk, cplx<R> Zc, cplx<R> wN) {
+  const cplx<R> cZc = conj(Zc);
+  const cplx<R> F = cadd(Zk, cZc), D = csub(Zk, cZc);
+  const cplx<R> t = cmul(D, wN);
   return {(R)0.5 * (F.x + t.y), (R)0.5 * (F.y - t.x)};
 }
 

@@ -4,7 +4,11 @@
 // One row belongs to one half-warp: lane l (0..15) holds Q values in
 // registers and the row is transformed by three Stockham passes
 //   radix Q (span 1), radix 4 (span Q), radix 4 (span 4 Q)
-// with the same butterfly map as fft_stage (fft.cuh).  Between passes the row
+// (Govindaraju et al., "High performance discrete Fourier transforms on graphics
+// processors", SC08): butterfly j of a pass of radix R and span Ns maps
+//   in : x[j + r H/R] * w^(r (j % Ns) H/(Ns R)),  r < R
+//   out: y[(j/Ns) Ns R + j % Ns + r Ns] = DFT_R(in)[r].
+// Between passes the row
 // goes through shared memory and only the half-warp synchronises
 // (__syncwarp), so rows of one CTA never wait for each other.  The radix-Q
 // butterfly is itself a two-factor Cooley-Tukey DFT in registers (Q = A B,
@@ -96,23 +100,6 @@ __device__ __forceinline__ void dft_q(cplx<float> (&v)[Q]) {
   else dft_ab<8, 3, INV>(v);
 }
 
-// Z[k] of the real-row synthesis (fft.cuh, c2r_pre) with the twiddle
-// wN = exp(-2 pi i k / N) already at hand.
-__device__ __forceinline__ cplx<float> c2r_pre_w(cplx<float> Xk, cplx<float> Xc, cplx<float> wN) {
-  const cplx<float> cXc = conj(Xc);
-  const cplx<float> F = cadd(Xk, cXc), D = csub(Xk, cXc);
-  const cplx<float> G = cmul(D, conj(wN));
-  return {F.x - G.y, F.y + G.x};
-}
-
-// X[k] of the real-row analysis (fft.cuh, r2c_post), wN = exp(-2 pi i k / N).
-__device__ __forceinline__ cplx<float> r2c_post_w(cplx<float> Zk, cplx<float> Zc, cplx<float> wN) {
-  const cplx<float> cZc = conj(Zc);
-  const cplx<float> F = cadd(Zk, cZc), D = csub(Zk, cZc);
-  const cplx<float> t = cmul(D, wN);
-  return {0.5f * (F.x + t.y), 0.5f * (F.y - t.x)};
-}
-
 // Twiddle tables of the two radix-4 passes, laid out [butterfly][r - 1] so
 // that the 16 lanes read words 3 apart (no bank conflicts):
 //   tw2[3 jm + r - 1] = w^(4 r jm), jm < Q;  tw3[3 j + r - 1] = w^(r j), j < 4 Q;
@@ -166,7 +153,7 @@ __device__ __forceinline__ void hw_row_fft(cplx<float>* row, int lane, unsigned 
         x.y = 0.f;
         xc = {0.f, 0.f};
       }
-      x = c2r_pre_w(x, xc, twN[k]);
+      x = c2r_pre(x, xc, twN[k]);
     }
     v[r] = x;
   }

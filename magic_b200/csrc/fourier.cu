@@ -56,9 +56,9 @@ __global__ void __launch_bounds__(kFftThreads, SH::kMax <= 12 ? 3 : 2)
         cplx<double>* z = buf + q * sh.S;
         const cplx<double> w = twN[k];
         const cplx<double> Xk = {xa[u].x, k ? xa[u].y : 0.0}, Xc = {xb[u].x, xb[u].y};
-        z[phi_slot(sh, k)] = c2r_pre_d(Xk, Xc, w);
+        z[phi_slot(sh, k)] = c2r_pre(Xk, Xc, w);
         if (k > 0 && 2 * k < H)  // exp(-2 pi i (H - k) / N) = -conj(w)
-          z[phi_slot(sh, H - k)] = c2r_pre_d(Xc, Xk, cplx<double>{-w.x, w.y});
+          z[phi_slot(sh, H - k)] = c2r_pre(Xc, Xk, cplx<double>{-w.x, w.y});
       }
     }
   }
@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(kFftThreads, SH::kMax <= 12 ? 3 : 2)
   for (int e = threadIdx.x; e < M * ncol; e += kFftThreads) {
     const int k = fdiv(e, rcpc), q = e - k * ncol;
     const cplx<double>* z = buf + q * sh.S;
-    const cplx<double> X = r2c_post_d(z[phi_slot(sh, k)], z[phi_slot(sh, k ? H - k : 0)], twN[k]);
+    const cplx<double> X = r2c_post(z[phi_slot(sh, k)], z[phi_slot(sh, k ? H - k : 0)], twN[k]);
     Fr[k * a.f_m + q] = make_double2(w * X.x, w * X.y);
   }
 }

@@ -44,7 +44,8 @@ __global__ void __launch_bounds__(kNlAnelThreads, 2) k_nl_anel_f64(NlAnelArgs a)
   phi_prefetch<NFI, T>(M, a.fs_m, at);
   const double* frow = at(row, r);
   phi_load_rows<NFI, T>(buf, sh, M, twN, [&](int k, int f) {
-    return __ldg(reinterpret_cast<const double2*>(frow + (int64_t)k * a.fs_m) + f);
+    const double2 x = __ldg(reinterpret_cast<const double2*>(frow + (int64_t)k * a.fs_m) + f);
+    return cplx<double>{x.x, x.y};
   });
   phi_inverse(buf, NFI, sh, tw1);
 

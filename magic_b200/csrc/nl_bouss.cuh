@@ -54,7 +54,8 @@ __global__ void __launch_bounds__(T, 512 / T) k_nl_bouss(NlBoussArgs a) {
   phi_prefetch<NFI, T>(M, pitch, at);
   const double* x0 = at(row, r);
   auto ldF = [&](int k, int f) {
-    return __ldg(reinterpret_cast<const double2*>(x0 + (int64_t)k * pitch) + f);
+    const double2 x = __ldg(reinterpret_cast<const double2*>(x0 + (int64_t)k * pitch) + f);
+    return cplx<double>{x.x, x.y};
   };
   phi_load_rows<NFI, T>(buf, sh, M, twN, ldF);
   phi_inverse(buf, NFI, sh, tw1);

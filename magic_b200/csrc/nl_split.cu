@@ -76,10 +76,16 @@ struct SplitFields {
   static constexpr int IV = MAG ? 6 : 0;
 };
 
-constexpr int kNlSplitThreads = 256;
-
-template <bool MAG, bool CHEM>
-__global__ void __launch_bounds__(kNlSplitThreads) k_nl_bouss_split(NlSplitArgs a) {
+// Row lengths without a half-warp form: block-wide Stockham passes (fft.cuh).  The
+// operations and their order are fixed: the Courant step of a boundary level is
+// the FP32 noise of a radial velocity that is zero there, and it goes into the
+// run's log, so a run must not see another rounding of it.  T threads and
+// `batch` rows per pass: seven rows of n_phi 192 are 84 radix-8 butterflies, which
+// left two thirds of 256 threads idle, two CTAs to an SM by their registers
+// (l_max 64, 33 levels: the whole stage 229 us, now 162; l_max 100, 65 levels, n_phi
+// 300: 816, now 579).
+template <bool MAG, bool CHEM, int T>
+__global__ void __launch_bounds__(T, 768 / T) k_nl_bouss_split(NlSplitArgs a, int batch) {
   using BF = SplitFields<MAG, CHEM>;
   constexpr int NFI = BF::NFI, NFO = BF::NFO;
   extern __shared__ __align__(16) float smemf[];
@@ -91,7 +97,7 @@ __global__ void __launch_bounds__(kNlSplitThreads) k_nl_bouss_split(NlSplitArgs 
   const int row = blockIdx.x, r = blockIdx.y;
   const int j = row >> 1;
   const float hs = (row & 1) ? -1.f : 1.f;  // north = sym + asym, south = sym - asym
-  cplx<float>* tws = buf + (BF::NB + kFftRowBatch) * stride;
+  cplx<float>* tws = buf + (BF::NB + batch) * stride;
   fft_twiddles_to_smem(tws, H, t.twiddle, t.fft_radix, t.fft_nstages);
   for (int i = threadIdx.x; i < NFI * stride; i += blockDim.x) buf[i] = {0.f, 0.f};
   __syncthreads();
@@ -103,7 +109,7 @@ __global__ void __launch_bounds__(kNlSplitThreads) k_nl_bouss_split(NlSplitArgs 
     buf[f * stride + pad16(k)] = {sy.x + hs * as.x, sy.y + hs * as.y};
   }
   __syncthreads();
-  for (int f = threadIdx.x / 32; f < NFI; f += kNlSplitThreads / 32)
+  for (int f = threadIdx.x / 32; f < NFI; f += T / 32)
     for (int k = threadIdx.x % 32; k <= H / 2; k += 32) {
       cplx<float>* rw = buf + f * stride;
       int kc = H - k;
@@ -120,7 +126,7 @@ __global__ void __launch_bounds__(kNlSplitThreads) k_nl_bouss_split(NlSplitArgs 
       }
     }
   __syncthreads();
-  fft_rows<true>(buf, buf + BF::NB * stride, NFI, H, stride, t.fft_radix, t.fft_nstages, tws);
+  fft_rows<true>(buf, buf + BF::NB * stride, NFI, batch, H, stride, t.fft_radix, t.fft_nstages, tws);
 
   const float or2 = (float)a.or2[r], or4 = (float)a.or4[r], ost2 = (float)t.ost2[row];
   const double orho1 = a.orho1[r], orho2 = a.orho2[r];
@@ -171,7 +177,7 @@ __global__ void __launch_bounds__(kNlSplitThreads) k_nl_bouss_split(NlSplitArgs 
   if (threadIdx.x == 0) atomicMax(&a.vh2max[r], (unsigned long long)__double_as_longlong(vmh + 0.0));
   if (r == 0 || r == a.n_r - 1) return;
   __syncthreads();
-  fft_rows<false>(buf, buf + BF::NB * stride, NFO, H, stride, t.fft_radix, t.fft_nstages, tws);
+  fft_rows<false>(buf, buf + BF::NB * stride, NFO, batch, H, stride, t.fft_radix, t.fft_nstages, tws);
   const float ws = (float)(t.wq[row] / N), wv = (float)(t.wq_v[row] / N);
   float* Gr = a.G + (int64_t)(row & 1) * a.g_h + (int64_t)j * a.g_j + (int64_t)(r - 1) * a.g_level;
   for (int e = threadIdx.x; e < M * NFO; e += blockDim.x) {
@@ -293,7 +299,7 @@ __global__ void __maxnreg__(72)
   for (int e = tid; e < M * NFO; e += T) {
     const int k = e / NFO, o = e - k * NFO;
     const cplx<float>* z = buf + o * S;
-    const cplx<float> X = r2c_post_w(z[hw_swz<Q>(k)], z[hw_swz<Q>((H - k) % H)], twN[k]);
+    const cplx<float> X = r2c_post(z[hw_swz<Q>(k)], z[hw_swz<Q>((H - k) % H)], twN[k]);
     const bool radial = (o == 0 || o == 3 || (MAG && o == 6) || (CHEM && o == (MAG ? 9 : 6)));
     const float w = radial ? ws : wv;
     reinterpret_cast<float2*>(Gr + k * a.g_m)[o] = make_float2(w * X.x, w * X.y);
@@ -315,6 +321,20 @@ static int launch_hw(const NlSplitArgs& a, cudaStream_t st) {
   return MT_OK;
 }
 
+template <bool MAG, bool CHEM, int T>
+static int launch_block(const NlSplitArgs& a, cudaStream_t st) {
+  using BF = SplitFields<MAG, CHEM>;
+  const int batch = a.t.n_phi <= 640 ? BF::NB : 7;  // all rows where they are short
+  const size_t sm = ((size_t)(BF::NB + batch) * padded_len(a.t.n_phi / 2) + a.t.n_phi / 2) *
+                    sizeof(cplx<float>);
+  auto kern = k_nl_bouss_split<MAG, CHEM, T>;
+  MT_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  dim3 grid(a.t.n_theta, a.n_r);
+  kern<<<grid, T, sm, st>>>(a, batch);
+  MT_CHECK_CUDA(cudaGetLastError());
+  return MT_OK;
+}
+
 template <bool MAG, bool CHEM>
 static int launch_t(const NlSplitArgs& a, cudaStream_t st) {
   switch (a.t.n_phi) {
@@ -324,15 +344,8 @@ static int launch_t(const NlSplitArgs& a, cudaStream_t st) {
     case 768: return launch_hw<MAG, CHEM, 24>(a, st);
     default: break;
   }
-  using BF = SplitFields<MAG, CHEM>;
-  size_t sm = ((size_t)(BF::NB + kFftRowBatch) * padded_len(a.t.n_phi / 2) + a.t.n_phi / 2) *
-              sizeof(cplx<float>);
-  auto kern = k_nl_bouss_split<MAG, CHEM>;
-  MT_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  dim3 grid(a.t.n_theta, a.n_r);
-  kern<<<grid, kNlSplitThreads, sm, st>>>(a);
-  MT_CHECK_CUDA(cudaGetLastError());
-  return MT_OK;
+  return a.t.n_phi <= 300 ? launch_block<MAG, CHEM, 128>(a, st)
+                          : launch_block<MAG, CHEM, 256>(a, st);
 }
 
 int launch_nl_bouss_split(bool mag, bool chem, const NlSplitArgs& a, cudaStream_t st) {

@@ -236,17 +236,19 @@ __device__ __forceinline__ void phi_outer_r(cplx<T>* buf, int nrows, const SH& s
 #pragma unroll
     for (int q = 0; q < R; ++q) v[q] = x[q * sh.P];
     if (INV) phi_dft<R, INV>(v);
-    // w^q, w = tw1's exp(-2 pi i j / H): read for q < 4 and multiples of four,
-    // one product (one rounding) for the others, 6 of 15 reads at R = 16
+    // w^q, w = tw1's exp(-2 pi i j / H): in FP64 read for q < 4 and multiples of
+    // four, one product (one rounding) for the others, 6 of 15 reads at R = 16;
+    // in FP32, where that rounding would show and the reads are half the size,
+    // all read
     cplx<T> wb[4];
 #pragma unroll
     for (int q = 1; q < R; ++q) {
       cplx<T> w;
-      if (q < 4 || q % 4 == 0) {
+      if (sizeof(T) == 4 || q < 4 || q % 4 == 0) {
         w = tw1[(q - 1) * sh.Ns + j];
         if (INV) w.y = -w.y;
         if (q < 4) wb[q] = w;
-        else wb[0] = w;
+        else if (q % 4 == 0) wb[0] = w;
       } else {
         w = cmul(wb[0], wb[q % 4]);
       }
@@ -357,24 +359,6 @@ __device__ __forceinline__ void phi_twiddles_to_smem(cplx<T>* tws, const SH& sh,
   }
 }
 
-// Z[k] of the real-row synthesis (c2r_pre) with wN = exp(-2 pi i k / N) at hand.
-template <typename T>
-__device__ __forceinline__ cplx<T> c2r_pre_d(cplx<T> Xk, cplx<T> Xc, cplx<T> wN) {
-  const cplx<T> cXc = conj(Xc);
-  const cplx<T> F = cadd(Xk, cXc), D = csub(Xk, cXc);
-  const cplx<T> G = cmul(D, conj(wN));
-  return {F.x - G.y, F.y + G.x};
-}
-
-// X[k] of the real-row analysis (r2c_post), wN = exp(-2 pi i k / N).
-template <typename T>
-__device__ __forceinline__ cplx<T> r2c_post_d(cplx<T> Zk, cplx<T> Zc, cplx<T> wN) {
-  const cplx<T> cZc = conj(Zc);
-  const cplx<T> F = cadd(Zk, cZc), D = csub(Zk, cZc);
-  const cplx<T> t = cmul(D, wN);
-  return {(T)0.5 * (F.x + t.y), (T)0.5 * (F.y - t.x)};
-}
-
 // The phases of a fused stage around the row FFTs (T = blockDim.x threads).
 
 // Asks the L2 for the rows that the CTA about to follow this one on its SM will
@@ -398,17 +382,17 @@ __device__ __forceinline__ void phi_prefetch(int M, int64_t pitch, At at) {
 // c2r_pre(X[H - k], X[k]).  kLd pairs per thread are loaded before any is
 // stored, so their HBM latencies overlap (the first round's also cover the
 // asynchronous copies of the twiddle tables).
-template <int NF, int T, class SH, typename Ld>
-__device__ __forceinline__ void phi_load_rows(cplx<double>* buf, const SH& sh, int M,
-                                              const cplx<double>* __restrict__ twN, Ld ld) {
+template <int NF, int T, class SH, typename R, typename Ld>
+__device__ __forceinline__ void phi_load_rows(cplx<R>* buf, const SH& sh, int M,
+                                              const cplx<R>* __restrict__ twN, Ld ld) {
   constexpr int kLd = 6;
   const int H = sh.H, total = (H / 2 + 1) * NF;
   for (int e0 = 0; e0 < total; e0 += kLd * T) {
-    double2 xa[kLd], xb[kLd];
+    cplx<R> xa[kLd], xb[kLd];
 #pragma unroll
     for (int u = 0; u < kLd; ++u) {
       const int e = e0 + u * T + (int)threadIdx.x, k = e / NF, f = e - k * NF;
-      xa[u] = xb[u] = make_double2(0.0, 0.0);
+      xa[u] = xb[u] = {(R)0, (R)0};
       if (e < total) {
         if (k < M) xa[u] = ld(k, f);
         if (k > 0 && H - k < M) xb[u] = ld(H - k, f);
@@ -422,12 +406,12 @@ __device__ __forceinline__ void phi_load_rows(cplx<double>* buf, const SH& sh, i
     for (int u = 0; u < kLd; ++u) {
       const int e = e0 + u * T + (int)threadIdx.x, k = e / NF, f = e - k * NF;
       if (e < total) {
-        cplx<double>* z = buf + f * sh.S;
-        const cplx<double> w = twN[k];
-        const cplx<double> Xk = {xa[u].x, k ? xa[u].y : 0.0}, Xc = {xb[u].x, xb[u].y};
-        z[phi_slot(sh, k)] = c2r_pre_d(Xk, Xc, w);
+        cplx<R>* z = buf + f * sh.S;
+        const cplx<R> w = twN[k];
+        const cplx<R> Xk = {xa[u].x, k ? xa[u].y : (R)0};
+        z[phi_slot(sh, k)] = c2r_pre(Xk, xb[u], w);
         if (k > 0 && 2 * k < H)  // exp(-2 pi i (H - k) / N) = -conj(w)
-          z[phi_slot(sh, H - k)] = c2r_pre_d(Xc, Xk, cplx<double>{-w.x, w.y});
+          z[phi_slot(sh, H - k)] = c2r_pre(xb[u], Xk, cplx<R>{-w.x, w.y});
       }
     }
   }
@@ -438,19 +422,19 @@ __device__ __forceinline__ void phi_load_rows(cplx<double>* buf, const SH& sh, i
 // phi_forward: a thread takes one component (real or imaginary part) of the
 // two elements g = 0, 1 of (p, s), which are two grid points after the F = 2
 // butterfly, and puts the outputs' butterfly in their place.
-template <int NFI, int NFO, int T, class SH, typename Fn>
-__device__ __forceinline__ void phi_points(cplx<double>* buf, const SH& sh, Fn& point) {
-  double* bd = reinterpret_cast<double*>(buf);
+template <int NFI, int NFO, int T, class SH, typename R, typename Fn>
+__device__ __forceinline__ void phi_points(cplx<R>* buf, const SH& sh, Fn& point) {
+  R* bd = reinterpret_cast<R*>(buf);
   const int total = 2 * sh.A * sh.B, S2 = 2 * sh.S, g = 2 * sh.B;
   for (int e = threadIdx.x; e < total; e += T) {
     const int u = e >> 1, s = sh.divA(u), p = u - s * sh.A;
-    double* x = bd + 2 * (p * sh.P + s) + (e & 1);
-    double v0[NFI], o0[NFO];
+    R* x = bd + 2 * (p * sh.P + s) + (e & 1);
+    R v0[NFI], o0[NFO];
     if (sh.F == 2) {
-      double v1[NFI], o1[NFO];
+      R v1[NFI], o1[NFO];
 #pragma unroll
       for (int f = 0; f < NFI; ++f) {
-        const double y0 = x[f * S2], y1 = x[f * S2 + g];
+        const R y0 = x[f * S2], y1 = x[f * S2 + g];
         v0[f] = y0 + y1;
         v1[f] = y0 - y1;
       }
@@ -472,17 +456,17 @@ __device__ __forceinline__ void phi_points(cplx<double>* buf, const SH& sh, Fn& 
 }
 
 // put(k, f, X[k]) for the half spectra k < M of the NF rows.
-template <int NF, int T, class SH, typename Put>
-__device__ __forceinline__ void phi_store_rows(const cplx<double>* buf, const SH& sh, int M,
-                                               const cplx<double>* __restrict__ twN, Put put) {
+template <int NF, int T, class SH, typename R, typename Put>
+__device__ __forceinline__ void phi_store_rows(const cplx<R>* buf, const SH& sh, int M,
+                                               const cplx<R>* __restrict__ twN, Put put) {
   constexpr int kSt = 4;  // outputs per thread whose shared-memory reads are issued together
   for (int e0 = threadIdx.x; e0 < M * NF; e0 += kSt * T) {
-    cplx<double> zk[kSt], zc[kSt], wn[kSt];
+    cplx<R> zk[kSt], zc[kSt], wn[kSt];
 #pragma unroll
     for (int u = 0; u < kSt; ++u) {
       const int e = e0 + u * T, k = e / NF, f = e - k * NF;
       if (e < M * NF) {
-        const cplx<double>* z = buf + f * sh.S;
+        const cplx<R>* z = buf + f * sh.S;
         zk[u] = z[phi_slot(sh, k)];
         zc[u] = z[phi_slot(sh, k ? sh.H - k : 0)];
         wn[u] = twN[k];
@@ -491,7 +475,7 @@ __device__ __forceinline__ void phi_store_rows(const cplx<double>* buf, const SH
 #pragma unroll
     for (int u = 0; u < kSt; ++u) {
       const int e = e0 + u * T, k = e / NF, f = e - k * NF;
-      if (e < M * NF) put(k, f, r2c_post_d(zk[u], zc[u], wn[u]));
+      if (e < M * NF) put(k, f, r2c_post(zk[u], zc[u], wn[u]));
     }
   }
 }
