@@ -40,11 +40,20 @@ __device__ __forceinline__ double2 load_term(const TermSrc& s, int64_t row, int6
   }
 }
 
+// Row strides of the staged tiles.  A fragment load reads 4 K rows x 8 columns (A
+// of the synthesis, B) or 8 rows x 4 K (A of the analysis) of doubles, served by
+// half-warps: four neighbours' rows must fall on different quarters of the 128
+// bytes, i.e. lie 32 bytes apart mod 128.  The K rows of one parity are two apart
+// in the synthesis (stride 2 mod 16 doubles, so SA = 34 and SB = 2 R + 2) and
+// consecutive in the analysis's B (4 mod 16: 2 R + 4).  At 64 bytes apart, which
+// took two passes, the FP64 stage at l_max 170 on 65 levels was 2.24 ms (now 2.16)
+// and the transforms of 37 columns at l_max 213 0.73 ms (now 0.685); the kernels
+// are bound by the FP64 tensor pipe and by these loads.
 template <class OP, int R>
 struct SynthCfg {
   static constexpr int TH = 32, KC = 16;
-  static constexpr int SA = 36;         // sA row stride (doubles): 16*SA = 64 mod 128 B
-  static constexpr int SB = 2 * R + 4;  // sB row stride (doubles)
+  static constexpr int SA = 34;         // sA row stride (doubles): rows 2 apart 32 mod 128 B
+  static constexpr int SB = 2 * R + 2;  // sB row stride (doubles), the same
   static constexpr int WC = R / 8;      // column tiles per warp
   static constexpr int NA = OP::NT * KC * TH / 256;                 // A elems / thread
   static constexpr int NB = (OP::NX * KC * R + 255) / 256;          // B elems / thread
@@ -189,7 +198,7 @@ template <class OP, int R>
 struct AnalCfg {
   static constexpr int TK = 64, KC = 16;
   static constexpr int SA = 18;         // sA row stride: rows 2 apart -> 32 B bank step
-  static constexpr int SB = 2 * R + 8;  // sB row stride: 8*SB = 64 mod 128 B
+  static constexpr int SB = 2 * R + 4;  // sB row stride: 8*SB = 32 mod 128 B
   static constexpr int WC = R / 4;
   static constexpr int NA = OP::NT * TK * KC / 256;
   static constexpr int NB = (OP::NX * KC * R + 255) / 256;
