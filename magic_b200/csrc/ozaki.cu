@@ -412,9 +412,11 @@ int ozaki_syn_total_chunks(const mt_plan* p) { return ((OzStore*)p->ozaki)->h_pr
 
 constexpr int kOzPackThreads = 256;
 
-__host__ __device__ inline int oz_stage_pitch(int stg_lev) { return 2 * kOzK * stg_lev + 1; }
+// staged slice: kOzK values of l - m (half a chunk of each parity), a ring of three
+constexpr int kOzSlices = 3;
+__host__ __device__ inline int oz_stage_pitch(int stg_lev) { return kOzK * stg_lev + 1; }
 __host__ __device__ inline size_t oz_syn_pack_smem(int narr, int stg_lev) {
-  return (size_t)narr * oz_stage_pitch(stg_lev) * 16 + 2 * kOzRows * sizeof(int);
+  return (size_t)kOzSlices * narr * oz_stage_pitch(stg_lev) * 16 + 2 * kOzRows * sizeof(int);
 }
 
 __host__ __device__ inline int64_t oz_syn_img_chunk(int64_t total_chunks, int rt, int prefix, int c,
@@ -445,9 +447,12 @@ __device__ __forceinline__ void cp_commit_wait_all() {
 
 // k_oz_syn_pack: block (row tile rt, order m).  Thread = (table q, parity p,
 // row pair): rows 2 pr, 2 pr + 1 are the real and imaginary rows of one field.
-// Pass 0 walks every chunk of 2 kOzK values of l - m and finds the largest
-// |value| of each (row, combo); pass 1 walks them again and writes the six
-// digit planes of every chunk at the row's scale.
+// Pass 0 walks the values of l - m and finds the largest |value| of each (row,
+// combo); pass 1 walks them again and writes the six digit planes of every
+// chunk at the row's scale.  The spectra arrive in slices of kOzK values by
+// asynchronous copies, two slices ahead of the one in use (one barrier per
+// slice); waiting for each 2 kOzK values in turn took 0.86 ms at l_max 255 on 97
+// levels, against 0.21 ms for its bytes (the stage there: 5.78 -> 5.74 ms).
 __global__ void __launch_bounds__(kOzPackThreads, 2) k_oz_syn_pack(OzSynArgs a) {
   extern __shared__ __align__(128) uint8_t smem[];
   const Tables& t = a.t;
@@ -460,11 +465,13 @@ __global__ void __launch_bounds__(kOzPackThreads, 2) k_oz_syn_pack(OzSynArgs a) 
   const int nlev = min(a.stg_lev, a.n_lev - lev0);
   const int pitch = oz_stage_pitch(a.stg_lev);
   double2* d = reinterpret_cast<double2*>(smem);
-  int* rexp_s = reinterpret_cast<int*>(smem + (size_t)a.narr * pitch * 16);  // [combo][row]
+  const int slice = a.narr * pitch;
+  int* rexp_s = reinterpret_cast<int*>(smem + (size_t)kOzSlices * slice * 16);  // [combo][row]
   const int qp = tid >> 6, row0 = 2 * (tid & 63);
   const int q = qp >> 1, p = qp & 1;
   const int combo = q == 0 ? p : 1 - p;
-  const int nch_all = (nlm + 2 * kOzK - 1) / (2 * kOzK);
+  const int nsl0 = (nlm + kOzK - 1) / kOzK;                     // slices with values
+  const int nsl1 = 2 * ((nlm + 2 * kOzK - 1) / (2 * kOzK));     // slices of whole chunks
   const int nch_combo = oz_syn_nch(nlm, combo);
   const double dm = (double)m;
   struct RowSrc {
@@ -488,39 +495,51 @@ __global__ void __launch_bounds__(kOzPackThreads, 2) k_oz_syn_pack(OzSynArgs a) 
     rs[h].ia = tm.ia * pitch + (lev - lev0);
     rs[h].ib = tm.ib * pitch + (lev - lev0);
   }
-  // value of row h at the i-th l - m of parity p in chunk c (staged)
-  auto value = [&](int h, int c, int i) -> double {
-    const int kk = 2 * i + p;  // l - m offset inside the staged chunk
-    const double l = (double)(m + 2 * kOzK * c + kk);
-    const double2 x = d[rs[h].ia + kk * a.stg_lev];
-    const double2 w = rs[h].cw != 0.0 ? d[rs[h].ib + kk * a.stg_lev] : make_double2(0.0, 0.0);
+  // value of row h at the i-th l - m of parity p in the staged slice sl
+  auto value = [&](int h, int sl, int i) -> double {
+    const int kk = 2 * i + p;  // l - m offset inside the slice
+    const double l = (double)(m + kOzK * sl + kk);
+    const double2* x = d + (sl % kOzSlices) * slice + kk * a.stg_lev;
+    const double2 xv = x[rs[h].ia];
+    const double2 w = rs[h].cw != 0.0 ? x[rs[h].ib] : make_double2(0.0, 0.0);
     const double mul = rs[h].o2 * (1.0 + rs[h].dl * (l * (l + 1.0) - 1.0));
-    const double xa = rs[h].cpart ? x.y : x.x, xb = rs[h].cpart ? w.y : w.x;
+    const double xa = rs[h].cpart ? xv.y : xv.x, xb = rs[h].cpart ? w.y : w.x;
     return rs[h].f * (mul * xa - rs[h].cw * xb);
   };
-  auto stage = [&](int c) {
-    __syncthreads();  // the staging buffer is free
-    for (int e = tid; e < 2 * kOzK * a.stg_lev; e += kOzPackThreads) {
-      const int kk = e / a.stg_lev, lvv = e - kk * a.stg_lev;
-      if (lvv >= nlev) continue;
-      const int k = 2 * kOzK * c + kk;
-      const int64_t off = (int64_t)(ls + min(k, nlm - 1)) * a.ld + lev0 + lvv;
-      const uint32_t bytes = k < nlm ? 16u : 0u;
-      for (int ia = 0; ia < a.narr; ++ia)
-        cp16_zfill(&d[ia * pitch + kk * a.stg_lev + lvv], a.arr[ia] + off, bytes);
+  // copies of slice sl (zeros past nlm), one commit group; nothing from nsl on
+  auto stage = [&](int sl, int nsl) {
+    if (sl < nsl) {
+      double2* dst = d + (sl % kOzSlices) * slice;
+      for (int e = tid; e < kOzK * a.stg_lev; e += kOzPackThreads) {
+        const int kk = e / a.stg_lev, lvv = e - kk * a.stg_lev;
+        if (lvv >= nlev) continue;
+        const int k = kOzK * sl + kk;
+        const int64_t off = (int64_t)(ls + min(k, nlm - 1)) * a.ld + lev0 + lvv;
+        const uint32_t bytes = k < nlm ? 16u : 0u;
+        for (int ia = 0; ia < a.narr; ++ia)
+          cp16_zfill(&dst[ia * pitch + kk * a.stg_lev + lvv], a.arr[ia] + off, bytes);
+      }
     }
-    cp_commit_wait_all();
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  // slice sl is complete and everyone is done with slice sl - 1, whose buffer
+  // takes slice sl + 2
+  auto next = [&](int sl, int nsl) {
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
     __syncthreads();
+    stage(sl + 2, nsl);
   };
   // pass 0: row maxima per combo; each (row, combo) gets contributions from
   // two threads (P of one parity, dP of the other), merged through shared memory
   double mx[2] = {0.0, 0.0};
-  for (int c = 0; c < nch_all; ++c) {
-    stage(c);
+  stage(0, nsl0);
+  stage(1, nsl0);
+  for (int sl = 0; sl < nsl0; ++sl) {
+    next(sl, nsl0);
 #pragma unroll 4
-    for (int i = 0; i < kOzK; ++i) {
-      mx[0] = fmax(mx[0], fabs(value(0, c, i)));
-      mx[1] = fmax(mx[1], fabs(value(1, c, i)));
+    for (int i = 0; i < kOzK / 2; ++i) {
+      mx[0] = fmax(mx[0], fabs(value(0, sl, i)));
+      mx[1] = fmax(mx[1], fabs(value(1, sl, i)));
     }
   }
   unsigned long long* rmax = reinterpret_cast<unsigned long long*>(smem);  // reuses staging
@@ -539,29 +558,29 @@ __global__ void __launch_bounds__(kOzPackThreads, 2) k_oz_syn_pack(OzSynArgs a) 
   }
   __syncthreads();
   const int ex[2] = {rexp_s[combo * kOzRows + row0], rexp_s[combo * kOzRows + row0 + 1]};
-  // pass 1: digit planes
-  for (int c = 0; c < nch_all; ++c) {
-    stage(c);
+  // pass 1: digit planes, a slice being half a chunk
+  stage(0, nsl1);
+  stage(1, nsl1);
+  for (int sl = 0; sl < nsl1; ++sl) {
+    next(sl, nsl1);
+    const int c = sl >> 1, half = sl & 1;
     if (c >= nch_combo) continue;
     uint8_t* dst = a.aimg + oz_syn_img_chunk(a.total_chunks, rt,
                                              a.z.syn_prefix[mc * 2 + combo], c, q) * kOzAChunk;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-#pragma unroll 1
-      for (int half = 0; half < 2; ++half) {
-        uint32_t w[4][kOzDigits];
+      uint32_t w[4][kOzDigits];
 #pragma unroll
-        for (int i4 = 0; i4 < 4; ++i4) {
-          double v4[4];
+      for (int i4 = 0; i4 < 4; ++i4) {
+        double v4[4];
 #pragma unroll
-          for (int b = 0; b < 4; ++b) v4[b] = value(h, c, 16 * half + 4 * i4 + b);
-          oz_digit_words(v4, ex[h], w[i4]);
-        }
-#pragma unroll
-        for (int s = 0; s < kOzDigits; ++s)
-          *reinterpret_cast<uint4*>(dst + s * kOzAPlane + oz_off(row0 + h, 16 * half)) =
-              make_uint4(w[0][s], w[1][s], w[2][s], w[3][s]);
+        for (int b = 0; b < 4; ++b) v4[b] = value(h, sl, 4 * i4 + b);
+        oz_digit_words(v4, ex[h], w[i4]);
       }
+#pragma unroll
+      for (int s = 0; s < kOzDigits; ++s)
+        *reinterpret_cast<uint4*>(dst + s * kOzAPlane + oz_off(row0 + h, 16 * half)) =
+            make_uint4(w[0][s], w[1][s], w[2][s], w[3][s]);
     }
   }
 }
