@@ -170,6 +170,28 @@ __device__ __forceinline__ double oz_combine_u(const uint32_t (&c)[kOzGroups][W]
   return fma(p1, 2097152.0, p2);
 }
 
+// The same sum through int32: adjacent groups pair up as C_g 2^7 + C_(g+1), three
+// integer multiply-adds in place of half of the conversions and FP64 operations.
+// |C_g| <= (g + 1) 2^12 n for n accumulated terms, so the largest pair,
+// (5 2^7 + 6) 2^12 n, fits for n <= kOzPairTerms; every step up to the last fma is
+// exact, so the result is oz_combine_u's bit for bit.
+constexpr int kOzPairTerms = 800;
+
+template <int W>
+__device__ __forceinline__ void oz_pair_groups(const uint32_t (&c)[kOzGroups][W],
+                                               uint32_t (&q)[3][W]) {
+#pragma unroll
+  for (int h = 0; h < 3; ++h)
+#pragma unroll
+    for (int i = 0; i < W; ++i) q[h][i] = c[2 * h][i] * 128u + c[2 * h + 1][i];
+}
+
+template <int W>
+__device__ __forceinline__ double oz_combine_q(const uint32_t (&q)[3][W], int i) {
+  const double lo = fma(oz_i2d(q[1][i]), 16384.0, oz_i2d(q[2][i]));  // below 2^45
+  return fma(oz_i2d(q[0][i]), 268435456.0, lo);
+}
+
 // Named barrier over `n` threads that also ANDs a predicate across them, so
 // that all participants take the same branch afterwards.
 __device__ __forceinline__ void named_bar_sync(int id, int n) {
@@ -612,9 +634,16 @@ struct OzSynSmem {
 // every K step into the ring, warp 1 lane 0 issues the MMAs of every step
 // (oz_mma_chunk: eight MMAs covering the 21 digit pairs) into the six group
 // accumulators (TMEM columns 64 g) and commits at the end of each half, warps
-// 2-9 drain the accumulators (one TMEM lane and 32 columns per thread): the
+// 2-17 drain the accumulators (one TMEM lane and 16 columns per thread): the
 // symmetric half into the stash, then with the antisymmetric half the north
-// and south rows into Fs, handing the accumulators back after each half.
+// and south rows into Fs.  With kPairs (at most kOzPairTerms terms per sum) a
+// thread's 96 accumulator words shrink to 48 pair words as they are read, so the
+// accumulators go back to the MMA warp before the FP64 arithmetic and the
+// stores, which then run beside the next half's MMAs; without, they go back
+// after them.  The drain of one half was as long as its MMAs, and they took turns:
+// the pair words here and in the analysis took the stage at l_max 255 on 97 levels
+// from 5.74 to 5.56 ms, the anelastic one at l_max 383 on 129 from 15.67 to 15.0.
+template <bool kPairs>
 __global__ void __launch_bounds__(kOzSynThreads, 1) k_oz_synth_gemm(OzSynArgs a) {
   extern __shared__ __align__(128) uint8_t smem[];
   const Tables& t = a.t;
@@ -770,33 +799,60 @@ __global__ void __launch_bounds__(kOzSynThreads, 1) k_oz_synth_gemm(OzSynArgs a)
         tc_fence_after();
         const uint32_t taddr =
             tbase + ((uint32_t)(32 * quarter) << 16) + kOzSynEpiCols * half;
-#pragma unroll 1
-        for (int c0 = 0; c0 < kOzSynEpiCols; c0 += 8) {
-          uint32_t cg[kOzGroups][8];
-#pragma unroll
-          for (int g = 0; g < kOzGroups; ++g)
-            tmem_ld8_i32_nowait(taddr + g * kOzSynN + c0, cg[g]);
-          tmem_wait_ld();
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int fe = __shfl_sync(0xffffffffu, fe_l, c0 + i);
-            const int col = kOzSynEpiCols * half + c0 + i;
-            const double v = oz_scale(oz_combine_u(cg, i), er + fe - 12 - 35);
-            double* st = stash + col * kOzRows + R0;  // this thread's own entry
-            if (combo == 0) {
-              *st = v;
-            } else {
-              const int th = it.tau * kOzSynN + col;
-              if (R < a.nrows && th < t.nhs) {
-                const double sy = *st;
-                north[(int64_t)th * a.fs_j + R] = sy + v;
-                south[(int64_t)th * a.fs_j + R] = sy - v;
-              }
+        // value v of this thread's column: the symmetric half waits in the stash,
+        // the antisymmetric one completes the north and south rows
+        auto put = [&](int c, double v) {
+          const int col = kOzSynEpiCols * half + c;
+          double* st = stash + col * kOzRows + R0;  // this thread's own entry
+          if (combo == 0) {
+            *st = v;
+          } else {
+            const int th = it.tau * kOzSynN + col;
+            if (R < a.nrows && th < t.nhs) {
+              const double sy = *st;
+              north[(int64_t)th * a.fs_j + R] = sy + v;
+              south[(int64_t)th * a.fs_j + R] = sy - v;
             }
           }
+        };
+        if constexpr (kPairs) {
+          static_assert(kOzSynEpiCols == 16, "two batches of eight columns");
+          uint32_t pq[2][3][8];
+#pragma unroll
+          for (int b = 0; b < 2; ++b) {
+            uint32_t cg[kOzGroups][8];
+#pragma unroll
+            for (int g = 0; g < kOzGroups; ++g)
+              tmem_ld8_i32_nowait(taddr + g * kOzSynN + 8 * b, cg[g]);
+            tmem_wait_ld();
+            oz_pair_groups(cg, pq[b]);
+          }
+          tc_fence_before();
+          mbar_arrive(tempty);
+#pragma unroll
+          for (int b = 0; b < 2; ++b)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const int fe = __shfl_sync(0xffffffffu, fe_l, 8 * b + i);
+              put(8 * b + i, oz_scale(oz_combine_q(pq[b], i), er + fe - 12 - 35));
+            }
+        } else {
+#pragma unroll 1
+          for (int c0 = 0; c0 < kOzSynEpiCols; c0 += 8) {
+            uint32_t cg[kOzGroups][8];
+#pragma unroll
+            for (int g = 0; g < kOzGroups; ++g)
+              tmem_ld8_i32_nowait(taddr + g * kOzSynN + c0, cg[g]);
+            tmem_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const int fe = __shfl_sync(0xffffffffu, fe_l, c0 + i);
+              put(c0 + i, oz_scale(oz_combine_u(cg, i), er + fe - 12 - 35));
+            }
+          }
+          tc_fence_before();
+          mbar_arrive(tempty);
         }
-        tc_fence_before();
-        mbar_arrive(tempty);
       }
     }
   }
@@ -824,13 +880,14 @@ int launch_oz_synth(const OzSynArgs& a, cudaStream_t st) {
   k_oz_syn_pack<<<dim3(ntiles, a.t.n_m), kOzPackThreads, pack_sm, st>>>(a);
   MT_CHECK_CUDA(cudaGetLastError());
   const size_t sm = OzSynSmem::total;
-  MT_CHECK_CUDA(cudaFuncSetAttribute(k_oz_synth_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)sm));
+  // a sum has one term per degree: P on one parity of l - m, dP on the other
+  auto gemm = a.t.l_max + 1 <= kOzPairTerms ? k_oz_synth_gemm<true> : k_oz_synth_gemm<false>;
+  MT_CHECK_CUDA(cudaFuncSetAttribute(gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   int dev = 0, nsm = 148;
   MT_CHECK_CUDA(cudaGetDevice(&dev));
   MT_CHECK_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   const int nitems = ntiles * a.z.nthtile * a.t.n_m;
-  k_oz_synth_gemm<<<std::min(nitems, nsm), kOzSynThreads, sm, st>>>(a);
+  gemm<<<std::min(nitems, nsm), kOzSynThreads, sm, st>>>(a);
   MT_CHECK_CUDA(cudaGetLastError());
   return MT_OK;
 }
@@ -966,6 +1023,7 @@ struct OzAnaSmem {
   static constexpr size_t total = bar_off + 8 * (2 * kOzStages + 3) + 16;
 };
 
+template <bool kPairs>
 __global__ void __launch_bounds__(kOzAnaThreads, 1) k_oz_anal_gemm(OzAnaArgs a) {
   extern __shared__ __align__(128) uint8_t smem[];
   const Tables& t = a.t;
@@ -1123,11 +1181,13 @@ __global__ void __launch_bounds__(kOzAnaThreads, 1) k_oz_anal_gemm(OzAnaArgs a) 
         for (int g = 0; g < kOzGroups; ++g)
           tmem_ld8_i32_nowait(taddr + (uint32_t)((qs * kOzGroups + g) * kOzAnaN + cs + c0), cg[g]);
         tmem_wait_ld();
+        uint32_t pq[3][8];
+        if constexpr (kPairs) oz_pair_groups(cg, pq);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const int fe = __shfl_sync(0xffffffffu, fe_l, c0 + i);
-          xch[(qs * kOzRows + R0) * kOzXS + cs + c0 + i] =
-              oz_scale(oz_combine_u(cg, i), er + fe - 12 - 35);
+          const double v = kPairs ? oz_combine_q(pq, i) : oz_combine_u(cg, i);
+          xch[(qs * kOzRows + R0) * kOzXS + cs + c0 + i] = oz_scale(v, er + fe - 12 - 35);
         }
       }
       tc_fence_before();
@@ -1202,13 +1262,14 @@ int launch_oz_anal(const OzAnaArgs& a, cudaStream_t st) {
   pack<<<dim3(ntiles * (kOzRows / rb), a.t.n_m), kOzPackThreads, psm, st>>>(a);
   MT_CHECK_CUDA(cudaGetLastError());
   const size_t sm = OzAnaSmem::total;
-  MT_CHECK_CUDA(cudaFuncSetAttribute(k_oz_anal_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)sm));
+  // a sum has one term per theta pair
+  auto gemm = a.t.nhs <= kOzPairTerms ? k_oz_anal_gemm<true> : k_oz_anal_gemm<false>;
+  MT_CHECK_CUDA(cudaFuncSetAttribute(gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   int dev = 0, nsm = 148;
   MT_CHECK_CUDA(cudaGetDevice(&dev));
   MT_CHECK_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   const int nitems = ntiles * 2 * a.z.nlt * a.t.n_m;
-  k_oz_anal_gemm<<<std::min(nitems, nsm), kOzAnaThreads, sm, st>>>(a);
+  gemm<<<std::min(nitems, nsm), kOzAnaThreads, sm, st>>>(a);
   MT_CHECK_CUDA(cudaGetLastError());
   return MT_OK;
 }
