@@ -624,9 +624,16 @@ __device__ __forceinline__ void solve_rows_to(const double* __restrict__ Ml, int
   __syncthreads();
 }
 
-template <bool kStaged, int kNt>
-__global__ void __launch_bounds__(Bounds<kStaged, kNt == 2 ? 3 : 2>::kThreads,
-                                  Bounds<kStaged, kNt == 2 ? 3 : 2>::kBlocks)
+// kBand: banded factors.  The solve is one warp's serial chain while the others
+// wait, so what counts is how many CTAs an SM holds, and compiled apart from the
+// tensor-pipe tile the registers allow more of them: four here (five spill) and
+// three in k_update_poloidal, against three and two in one kernel with the dense
+// solve.  All updates of a step at l_max 255 on 97 finite-difference levels: 1061
+// -> 950 us (five CTAs here: 1244; two in k_update_poloidal: 962).
+// Otherwise a dense solve with kNt n-tiles per warp.
+template <bool kStaged, int kNt, bool kBand>
+__global__ void __launch_bounds__(Bounds<kStaged, 2>::kThreads,
+                                  Bounds<kStaged, kBand ? 4 : kNt == 2 ? 3 : 2>::kBlocks)
     k_update_field(UsArgs a) {
   extern __shared__ __align__(16) double2 usbuf[];
   __shared__ int lm_row[16];
@@ -635,20 +642,19 @@ __global__ void __launch_bounds__(Bounds<kStaged, kNt == 2 ? 3 : 2>::kThreads,
   const int nrow = cta_rows(mc0, rows, l, a.minc, a.n_m);
   if (nrow == 0) return;
   double2* f = usbuf;                           // [rows][fs]: rhs, then x
-  double* mbuf = (double*)(usbuf + rows * fs);  // staged: [2][kKc][ldm]
-  const bool band = a.band.abd != nullptr;
-  const double* Ml = band ? nullptr : a.mt + (int64_t)l * n_r * ldm;
-  if constexpr (kStaged)
-    if (!band) stage_chunk(Ml, n_r, ldm, 0, mbuf);
-  const BandView bv = band ? stage_band(a.band, l, n_r, mbuf) : a.band;
+  double* mbuf = (double*)(usbuf + rows * fs);  // dense: [2][kKc][ldm]; band: the factors
+  const double* Ml = kBand ? nullptr : a.mt + (int64_t)l * n_r * ldm;
+  if constexpr (kStaged && !kBand) stage_chunk(Ml, n_r, ldm, 0, mbuf);
+  BandView bv = a.band;
+  if constexpr (kBand) bv = stage_band(a.band, l, n_r, mbuf);
   if (threadIdx.x < rows)
     lm_row[threadIdx.x] = threadIdx.x < nrow
         ? a.lstart[mc0 + threadIdx.x] + (l - (mc0 + threadIdx.x) * a.minc) : 0;
   __syncthreads();
-  build_rhs<false, 3>(a, l, rows, nrow, lm_row, f);
+  build_rhs<false, kBand ? 2 : 3>(a, l, rows, nrow, lm_row, f);
   __syncthreads();
   const Slot s = slot_of(n_r, a.groups);
-  if (band) {
+  if constexpr (kBand) {
     band_solve(bv, l, n_r, fs, f, nrow, mc0);
     store_rows(f, fs, n_r, nrow, lm_row, a.x, a.ld);
   } else {
@@ -889,8 +895,9 @@ struct PwArgs {
 // Double-curl poloidal update (magic_torch/update_w_doublecurl.py:393-483):
 // same tiling as k_update_field; the CTA holding (l, m) = (0, 0) also solves
 // the l = 0 pressure (update_wp.py:173-194).
-template <bool kStaged, int kNt>
-__global__ void __launch_bounds__(Bounds<kStaged, 2>::kThreads, Bounds<kStaged, 2>::kBlocks)
+template <bool kStaged, int kNt, bool kBand>
+__global__ void __launch_bounds__(Bounds<kStaged, 2>::kThreads,
+                                  Bounds<kStaged, kBand ? 3 : 2>::kBlocks)
     k_update_poloidal(PwArgs a) {
   extern __shared__ __align__(16) double2 pwbuf[];
   __shared__ int lm_row[16];
@@ -901,11 +908,10 @@ __global__ void __launch_bounds__(Bounds<kStaged, 2>::kThreads, Bounds<kStaged, 
   double2* f = pwbuf;                 // [rows][fs]: rhs, then w
   double2* dd = pwbuf + rows * fs;    // [rows][fs]: D2 w
   double* mbuf = (double*)(pwbuf + 2 * rows * fs);
-  const bool band = a.band.abd != nullptr;
-  const double* Ml = band ? nullptr : a.mt + (int64_t)l * n_r * ldm;
-  if constexpr (kStaged)
-    if (!band) stage_chunk(Ml, n_r, ldm, 0, mbuf);
-  const BandView bv = band ? stage_band(a.band, l, n_r, mbuf) : a.band;
+  const double* Ml = kBand ? nullptr : a.mt + (int64_t)l * n_r * ldm;
+  if constexpr (kStaged && !kBand) stage_chunk(Ml, n_r, ldm, 0, mbuf);
+  BandView bv = a.band;
+  if constexpr (kBand) bv = stage_band(a.band, l, n_r, mbuf);
   const double2 zero = {0.0, 0.0};
   const double dL = (double)l * (l + 1.0);
   if (threadIdx.x < rows)
@@ -916,7 +922,7 @@ __global__ void __launch_bounds__(Bounds<kStaged, 2>::kThreads, Bounds<kStaged, 
   build_rhs<true, 2>(a, l, rows, nrow, lm_row, f);
   __syncthreads();
   const Slot s = slot_of(n_r, a.groups);
-  if (band) {
+  if constexpr (kBand) {
     band_solve(bv, l, n_r, fs, f, nrow, mc0);
     store_rows(f, fs, n_r, nrow, lm_row, a.w, a.ld);
   } else {
@@ -1758,8 +1764,10 @@ int mt_update_field(const mt_plan* p, int n_r, const mt_field_update* u, const m
              "tile shape does not cover n_r");
   a.groups = t.groups;
   a.fs = t.fs;
-  auto kern = !t.staged ? k_update_field<false, 2>
-                        : (t.nt == 2 ? k_update_field<true, 2> : k_update_field<true, 4>);
+  auto kern = solve->abd ? (t.staged ? k_update_field<true, 2, true> : k_update_field<false, 2, true>)
+              : !t.staged ? k_update_field<false, 2, false>
+              : t.nt == 2 ? k_update_field<true, 2, false>
+                          : k_update_field<true, 4, false>;
   MT_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t.smem));
   kern<<<t.grid, t.threads, t.smem, (cudaStream_t)stream>>>(a);
   MT_CHECK_CUDA(cudaGetLastError());
@@ -1848,8 +1856,11 @@ int mt_update_poloidal(const mt_plan* p, int n_r, const mt_poloidal_update* u,
              "tile shape does not cover n_r");
   a.groups = t.groups;
   a.fs = t.fs;
-  auto kern = !t.staged ? k_update_poloidal<false, 2>
-                        : (t.nt == 2 ? k_update_poloidal<true, 2> : k_update_poloidal<true, 4>);
+  auto kern =
+      solve->abd ? (t.staged ? k_update_poloidal<true, 2, true> : k_update_poloidal<false, 2, true>)
+      : !t.staged ? k_update_poloidal<false, 2, false>
+      : t.nt == 2 ? k_update_poloidal<true, 2, false>
+                  : k_update_poloidal<true, 4, false>;
   MT_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t.smem));
   kern<<<t.grid, t.threads, t.smem, (cudaStream_t)stream>>>(a);
   MT_CHECK_CUDA(cudaGetLastError());
