@@ -12,10 +12,16 @@
 namespace mt {
 
 constexpr int kColsPerCta = 8;  // real columns (grid rows) per CTA
-constexpr int kFftThreads = 256;
 
-template <class SH>
-__global__ void __launch_bounds__(kFftThreads, SH::kMax <= 12 ? 3 : 2)
+// Threads of a CTA: 256; 128, and so twice the CTAs an SM, for the largest
+// radices on at most kFewCols columns, where a step has too few transforms for
+// 256 threads (n_phi 250, 3 columns: 75 and 15) and the registers of a radix-25
+// transform allow two CTAs of that size only: a round trip of 3 columns at l_max
+// 327, minc 4 takes 173 us with 256 threads, 165 with 128.
+constexpr int kFftThreads = 256, kFewThreads = 128, kFewCols = 4;
+
+template <class SH, int T>
+__global__ void __launch_bounds__(T, T == kFewThreads ? 4 : SH::kMax <= 12 ? 3 : 2)
     k_fourier_to_grid(ToGridArgs a) {
   extern __shared__ double smem[];
   cplx<double>* buf = reinterpret_cast<cplx<double>*>(smem);
@@ -34,11 +40,11 @@ __global__ void __launch_bounds__(kFftThreads, SH::kMax <= 12 ? 3 : 2)
   // at k >= M (and X[H] = 0: 2 (n_m - 1) < N), kLd pairs in flight per thread
   constexpr int kLd = 4;
   const int total = (H / 2 + 1) * ncol;
-  for (int e0 = 0; e0 < total; e0 += kLd * kFftThreads) {
+  for (int e0 = 0; e0 < total; e0 += kLd * T) {
     double2 xa[kLd], xb[kLd];
 #pragma unroll
     for (int u = 0; u < kLd; ++u) {
-      const int e = e0 + u * kFftThreads + threadIdx.x, k = fdiv(e, rcp), q = e - k * ncol;
+      const int e = e0 + u * T + threadIdx.x, k = fdiv(e, rcp), q = e - k * ncol;
       xa[u] = xb[u] = make_double2(0.0, 0.0);
       if (e < total) {
         if (k < M) xa[u] = __ldg(&Fr[k * a.f_m + q]);
@@ -51,7 +57,7 @@ __global__ void __launch_bounds__(kFftThreads, SH::kMax <= 12 ? 3 : 2)
     }
 #pragma unroll
     for (int u = 0; u < kLd; ++u) {
-      const int e = e0 + u * kFftThreads + threadIdx.x, k = fdiv(e, rcp), q = e - k * ncol;
+      const int e = e0 + u * T + threadIdx.x, k = fdiv(e, rcp), q = e - k * ncol;
       if (e < total) {
         cplx<double>* z = buf + q * sh.S;
         const cplx<double> w = twN[k];
@@ -66,7 +72,7 @@ __global__ void __launch_bounds__(kFftThreads, SH::kMax <= 12 ? 3 : 2)
   phi_inverse(buf, ncol, sh, tw1);
   // one warp per row; lanes take consecutive complex points n = p + A s < A B
   const int lane = threadIdx.x & 31, AB = sh.A * sh.B;
-  for (int q = threadIdx.x >> 5; q < ncol; q += kFftThreads / 32) {
+  for (int q = threadIdx.x >> 5; q < ncol; q += T / 32) {
     const int c = col0 + q, f = c / a.B, b = c - f * a.B;
     double* dst = a.out[f] + ((int64_t)b * nt + row) * N;
     const bool wide = (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
@@ -92,8 +98,8 @@ __global__ void __launch_bounds__(kFftThreads, SH::kMax <= 12 ? 3 : 2)
   }
 }
 
-template <class SH>
-__global__ void __launch_bounds__(kFftThreads, SH::kMax <= 12 ? 3 : 2)
+template <class SH, int T>
+__global__ void __launch_bounds__(T, T == kFewThreads ? 4 : SH::kMax <= 12 ? 3 : 2)
     k_grid_to_fourier(ToFourierArgs a) {
   extern __shared__ double smem[];
   cplx<double>* buf = reinterpret_cast<cplx<double>*>(smem);
@@ -107,7 +113,7 @@ __global__ void __launch_bounds__(kFftThreads, SH::kMax <= 12 ? 3 : 2)
   cplx<double>* twN = tw1 + (sh.A - 1) * sh.Ns;
   phi_twiddles_to_smem(tw1, sh, t);
   const int lane = threadIdx.x & 31, AB = sh.A * sh.B;
-  for (int q = threadIdx.x >> 5; q < ncol; q += kFftThreads / 32) {
+  for (int q = threadIdx.x >> 5; q < ncol; q += T / 32) {
     const int c = col0 + q, f = c / a.B, b = c - f * a.B;
     const double2* src =
         reinterpret_cast<const double2*>(a.in[f] + ((int64_t)b * nt + row) * N);
@@ -132,7 +138,7 @@ __global__ void __launch_bounds__(kFftThreads, SH::kMax <= 12 ? 3 : 2)
   double2* Fr = a.F + (int64_t)row * a.f_row + col0;
   const float rcpc = 1.0f / (float)ncol;
 #pragma unroll 4
-  for (int e = threadIdx.x; e < M * ncol; e += kFftThreads) {
+  for (int e = threadIdx.x; e < M * ncol; e += T) {
     const int k = fdiv(e, rcpc), q = e - k * ncol;
     const cplx<double>* z = buf + q * sh.S;
     const cplx<double> X = r2c_post(z[phi_slot(sh, k)], z[phi_slot(sh, k ? H - k : 0)], twN[k]);
@@ -144,24 +150,24 @@ static size_t fft_smem(const Tables& t) {
   return ((size_t)kColsPerCta * phi_row_len(t) + phi_tw_len(t)) * sizeof(double2);
 }
 
-template <int kMax>
+template <int kMax, int T = kFftThreads>
 static int launch_to_grid(const ToGridArgs& a, cudaStream_t st) {
   const size_t sm = fft_smem(a.t);
-  auto kern = k_fourier_to_grid<PhiShapeRt<kMax>>;
+  auto kern = k_fourier_to_grid<PhiShapeRt<kMax>, T>;
   MT_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   dim3 grid((a.ncols + kColsPerCta - 1) / kColsPerCta, a.t.n_theta);
-  kern<<<grid, kFftThreads, sm, st>>>(a);
+  kern<<<grid, T, sm, st>>>(a);
   MT_CHECK_CUDA(cudaGetLastError());
   return MT_OK;
 }
 
-template <int kMax>
+template <int kMax, int T = kFftThreads>
 static int launch_to_fourier(const ToFourierArgs& a, cudaStream_t st) {
   const size_t sm = fft_smem(a.t);
-  auto kern = k_grid_to_fourier<PhiShapeRt<kMax>>;
+  auto kern = k_grid_to_fourier<PhiShapeRt<kMax>, T>;
   MT_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   dim3 grid((a.ncols + kColsPerCta - 1) / kColsPerCta, a.t.n_theta);
-  kern<<<grid, kFftThreads, sm, st>>>(a);
+  kern<<<grid, T, sm, st>>>(a);
   MT_CHECK_CUDA(cudaGetLastError());
   return MT_OK;
 }
@@ -169,13 +175,16 @@ static int launch_to_fourier(const ToFourierArgs& a, cudaStream_t st) {
 int launch_fourier_to_grid(const ToGridArgs& a, cudaStream_t st) {
   const int r = phi_max_radix(a.t);
   if (r <= 12) return launch_to_grid<12>(a, st);
-  return r <= 18 ? launch_to_grid<18>(a, st) : launch_to_grid<27>(a, st);
+  if (r <= 18) return launch_to_grid<18>(a, st);
+  return a.ncols <= kFewCols ? launch_to_grid<27, kFewThreads>(a, st) : launch_to_grid<27>(a, st);
 }
 
 int launch_grid_to_fourier(const ToFourierArgs& a, cudaStream_t st) {
   const int r = phi_max_radix(a.t);
   if (r <= 12) return launch_to_fourier<12>(a, st);
-  return r <= 18 ? launch_to_fourier<18>(a, st) : launch_to_fourier<27>(a, st);
+  if (r <= 18) return launch_to_fourier<18>(a, st);
+  return a.ncols <= kFewCols ? launch_to_fourier<27, kFewThreads>(a, st)
+                             : launch_to_fourier<27>(a, st);
 }
 
 // Largest n_phi that the row FFTs' two radices cover (phi_fft.cuh).
