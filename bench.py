@@ -194,7 +194,7 @@ class ClockSampler:
 # full-set capture of the same kernel at l_max = 255, n_r = 17, per Fourier row moved (13 fields x n_r in, 9 fields x (n_r - 2) out); traffic grows
 # in proportion to the rows, so the full-size launch is scaled by its row count.
 NCU_PHI_TRAFFIC = {"split": (230.161408e6 + 104.267520e6) / (13 * 17 + 9 * 15),
-                   # the FP64 phi kernel of the digit-split stage (k_nl_bouss_w64)
+                   # the FP64 phi kernel of the digit-split stage (k_nl_bouss)
                    "ozaki": (347.744000e6 + 178.849280e6) / (13 * 17 + 9 * 15)}
 # warp instructions of the same launch (smsp__inst_executed.sum), per Fourier row
 NCU_PHI_INST = {"split": 184287744.0 / (13 * 17 + 9 * 15),
@@ -302,8 +302,7 @@ def run_anel(args, rank, world):
     perturbations |c_lm| ~ 1e-3 (l+1)^-2), through magic_b200.step.AnelasticStep
     with the stage of --precision (default the fused digit-split stage), beside
     the other two (unless --no-alt): the fused split-precision stage and the
-    FP64 stage (composed from the FP64 transform kernels as the reference
-    composes it), all with the same FP64 solves; device-timed with the state resident (2.9 GB of spectral
+    FP64 stage (DMMA contractions and the FP64 phi kernel), all with the same FP64 solves; device-timed with the state resident (2.9 GB of spectral
     arrays, larger than L2)."""
     from magic_b200.step import AnelasticStep
 
@@ -342,7 +341,7 @@ def run_anel(args, rank, world):
     what = {"split": "the fused split-precision stage (bf16x3 tcgen05 GEMMs, FP32 phi stage)",
             "ozaki": "the fused digit-split stage (int8 digit-plane GEMMs, FP64 phi stage; "
                      "~1e-12 of scale)",
-            "fp64": "the FP64 stage (composed from the FP64 transform kernels)"}
+            "fp64": "the fused FP64 stage (DMMA contractions, FP64 phi kernel)"}
     alts = {}
     for prec in ([] if args.no_alt else [q for q in ("fp64", "split", "ozaki") if q != main]):
         sta = build(prec)

@@ -232,8 +232,7 @@ MT_API int mt_nl_bouss(const mt_plan* plan, int n_r, const mt_bouss_in* in,
  * and Courant maxima in the phi stage, Legendre analysis of the bulk levels.
  * Requires a plan created with MT_PREC_SPLIT (tcgen05 bf16x3 GEMMs, FP32 phi
  * stage) or MT_PREC_OZAKI (int8 digit-plane GEMMs, FP64 phi stage, ~1e-12 of
- * scale); FP64 plans compose the drop-in transforms and mt_get_nl_anel
- * exactly as radial_loop_anel does.  The FP64 phi stage keeps the rows of
+ * scale); FP64 plans use mt_nl_anel_f64 below.  The FP64 phi stage keeps the rows of
  * one (theta row, level) in shared memory; where they would not fit (no plan
  * within the n_phi limit of mt_plan_create) mt_nl_anel_workspace returns 0
  * and mt_nl_anel MT_ERR_UNSUPPORTED.
@@ -261,6 +260,14 @@ typedef struct {
 
 MT_API size_t mt_nl_anel_workspace(const mt_plan* plan, int n_r, int l_mag, int l_chem);
 MT_API int mt_nl_anel(const mt_plan* plan, int n_r, const mt_anel_in* in,
+               const mt_anel_out* out, const mt_anel_stage_params* p, double* dtrkc,
+               double* dthkc, void* work, size_t work_bytes, void* stream);
+
+/* The same stage on a MT_PREC_FP64 plan: FP64 (DMMA) contractions and the FP64
+ * phi stage, grids never in device memory.  Also writes zeros to columns 0 and
+ * n_r-1 of the outputs. */
+MT_API size_t mt_nl_anel_f64_workspace(const mt_plan* plan, int n_r, int l_mag, int l_chem);
+MT_API int mt_nl_anel_f64(const mt_plan* plan, int n_r, const mt_anel_in* in,
                const mt_anel_out* out, const mt_anel_stage_params* p, double* dtrkc,
                double* dthkc, void* work, size_t work_bytes, void* stream);
 

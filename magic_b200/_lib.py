@@ -169,6 +169,9 @@ _PROTOS = {
     "mt_nl_anel_workspace": (C.c_size_t, [C.c_void_p, C.c_int, C.c_int, C.c_int]),
     "mt_nl_anel": (C.c_int, [C.c_void_p, C.c_int, C.POINTER(AnelIn), C.POINTER(AnelOut),
                              C.POINTER(AnelStageParams), _dp, _dp, _dp, C.c_size_t, _dp]),
+    "mt_nl_anel_f64_workspace": (C.c_size_t, [C.c_void_p, C.c_int, C.c_int, C.c_int]),
+    "mt_nl_anel_f64": (C.c_int, [C.c_void_p, C.c_int, C.POINTER(AnelIn), C.POINTER(AnelOut),
+                                 C.POINTER(AnelStageParams), _dp, _dp, _dp, C.c_size_t, _dp]),
     "mt_radial_op_create": (C.c_int, [C.c_int, C.POINTER(C.c_double), C.POINTER(C.c_void_p)]),
     "mt_radial_op_create_dct1": (C.c_int, [C.c_int, C.POINTER(C.c_void_p)]),
     "mt_radial_op_destroy": (C.c_int, [C.c_void_p]),

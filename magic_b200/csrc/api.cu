@@ -1366,6 +1366,158 @@ static int nl_anel_split_t(const mt_plan* p, int n_r, const mt_anel_in* in,
   return launch_courant_finish(n_r, mx, mx + n_r, q->delxr2, q->delxh2, dtrkc, dthkc, st);
 }
 
+// Arguments of the anelastic phi stages that do not depend on the row layout.
+static NlAnelArgs anel_phi_args(const mt_plan* p, int n_r, bool mag, const mt_anel_stage_params* q,
+                                unsigned long long* mx) {
+  NlAnelArgs nl{};
+  nl.t = p->tab;
+  nl.n_r = n_r;
+  nl.r = q->r;
+  nl.or1 = q->or1;
+  nl.or2 = q->or2;
+  nl.or4 = q->or4;
+  nl.beta = q->beta;
+  nl.orho1 = q->orho1;
+  nl.orho2 = q->orho2;
+  nl.otemp1 = q->otemp1;
+  nl.visc = q->visc;
+  nl.lambda_ = q->lambda_;
+  nl.delxr2 = q->delxr2;
+  nl.delxh2 = q->delxh2;
+  nl.LFfac = q->LFfac;
+  nl.ViscHeatFac = q->ViscHeatFac;
+  nl.OhmLossFac = mag ? q->OhmLossFac : 0.0;
+  nl.cour_mode = mag ? q->cour_mode : 0;
+  nl.cf2 = q->courfac * q->courfac;
+  nl.af2 = q->alffac * q->alffac;
+  const double h = 0.5 * (1.0 + q->opm);
+  nl.valfac = h * h;
+  nl.vr2max = mx;
+  nl.vh2max = mx + n_r;
+  return nl;
+}
+
+// Fused anelastic stage in FP64: two or three synthesis launches (SynAnelVel,
+// SynAnelDr, the magnetic groups) into FP64 Fourier rows F[m][theta row][level,
+// field], the phi stage k_nl_anel_f64, and the analysis launches of its products.
+// Grids never reach HBM: composed from the drop-in transforms the stage writes
+// and reads back 19 grids in and 13 out: 1.66 ms at l_max 127 on 65 levels, 0.4 ms
+// of it zero fills and copies between grids, against 1.09 ms here.
+template <bool MAG, bool CHEM>
+static int nl_anel_f64_t(const mt_plan* p, int n_r, const mt_anel_in* in, const mt_anel_out* out,
+                         const mt_anel_stage_params* q, double* dtrkc, double* dthkc, void* work,
+                         cudaStream_t st) {
+  const int nfi = anel_nfi(MAG, CHEM), nfo = anel_nfo(MAG, CHEM);
+  char* w = (char*)work;
+  double2* F = (double2*)w;
+  w += fourier_bytes(p, (int64_t)n_r * nfi);
+  double2* G = (double2*)w;
+  w += fourier_bytes(p, (int64_t)(n_r - 2) * nfo);
+  unsigned long long* mx = (unsigned long long*)w;
+  auto c = [](const double* x) { return (const double2*)x; };
+  const int64_t f_row = (int64_t)n_r * nfi, f_m = (int64_t)p->n_theta * f_row;
+  const int64_t g_row = (int64_t)(n_r - 2) * nfo, g_m = (int64_t)p->n_theta * g_row;
+  auto synth_args = [&](auto& s, int field0) {
+    s.t = p->tab;
+    s.ld = in->ld;
+    s.ncols = n_r;
+    s.or2 = q->or2;
+    s.F = F + field0;
+    s.f_row = f_row;
+    s.f_m = f_m;
+    s.col_f = 1;
+    s.col_c = nfi;
+  };
+  {
+    SynthArgs<4> s{};
+    synth_args(s, 0);
+    s.src[0] = {c(in->w), nullptr, kDlh};
+    s.src[1] = {c(in->dw), nullptr, kRaw};
+    s.src[2] = {c(in->z), nullptr, kRaw};
+    s.src[3] = {c(in->z), nullptr, kDlh};
+    MT_TRY((launch_synth_f64<SynAnelVel, 8>(s, st)));
+  }
+  {
+    using SO = SynAnelDr<CHEM ? 2 : 1>;
+    SynthArgs<SO::NX> s{};
+    synth_args(s, 0);
+    s.src[0] = {c(in->dw), nullptr, kDlh};
+    s.src[1] = {c(in->ddw), nullptr, kRaw};
+    s.src[2] = {c(in->dz), nullptr, kRaw};
+    s.src[3] = {c(in->s), nullptr, kRaw};
+    if (CHEM) s.src[SO::NX - 1] = {c(in->xi), nullptr, kRaw};
+    MT_TRY((launch_synth_f64<SO, 8>(s, st)));
+  }
+  if (MAG) {
+    SynthArgs<6> s{};
+    synth_args(s, 12 + (CHEM ? 1 : 0));
+    s.src[0] = {c(in->b), nullptr, kDlh};
+    s.src[1] = {c(in->db), nullptr, kRaw};
+    s.src[2] = {c(in->aj), nullptr, kRaw};
+    s.src[3] = {c(in->aj), nullptr, kDlh};
+    s.src[4] = {c(in->dj), nullptr, kRaw};
+    s.src[5] = {c(in->b), c(in->ddb), kCurlT};
+    MT_TRY((launch_synth_f64<SynGroups<2, 0>, 8>(s, st)));
+  }
+  MT_CHECK_CUDA(cudaMemsetAsync(mx, 0, 2 * n_r * sizeof(unsigned long long), st));
+  NlAnelArgs nl = anel_phi_args(p, n_r, MAG, q, mx);
+  // interleaved theta rows: a hemisphere's rows are two apart (strides in doubles)
+  nl.Fs64 = (const double*)F;
+  nl.fs_m = 2 * f_m;
+  nl.fs_c = 2 * f_row;
+  nl.fs_j = 4 * f_row;
+  nl.G64 = (double*)G;
+  nl.g_m = 2 * g_m;
+  nl.g_h = 2 * g_row;
+  nl.g_j = 4 * g_row;
+  nl.g_level = 2 * nfo;
+  MT_TRY(launch_nl_anel_f64(MAG, CHEM, nl, st));
+  auto anal_args = [&](auto& a, int field0) {
+    a.t = p->tab;
+    a.F = G + field0;
+    a.f_m = g_m;
+    a.f_row = g_row;
+    a.col_x = 1;
+    a.col_c = nfo;
+    a.ncols = n_r - 2;
+    a.ld = out->ld;
+    a.out_col0 = 1;
+    a.zero_ends = 1;
+  };
+  {
+    AnalArgs<6, 5> a{};
+    anal_args(a, 0);
+    a.out[0] = (double2*)out->Advr;
+    a.out[1] = (double2*)out->Advt;
+    a.out[2] = (double2*)out->Advp;
+    a.out[3] = (double2*)out->VSr;
+    a.out[4] = (double2*)out->VSt;
+    MT_TRY((launch_anal_f64<AnaGroups<1, 2>, 8>(a, st)));
+  }
+  if (MAG) {
+    AnalArgs<3, 3> a{};
+    anal_args(a, 6);
+    a.out[0] = (double2*)out->VxBr;
+    a.out[1] = (double2*)out->VxBt;
+    a.out[2] = (double2*)out->VxBp;
+    MT_TRY((launch_anal_f64<AnaGroups<1, 0>, 8>(a, st)));
+  }
+  if (CHEM) {
+    AnalArgs<3, 2> a{};
+    anal_args(a, MAG ? 9 : 6);
+    a.out[0] = (double2*)out->VXir;
+    a.out[1] = (double2*)out->VXit;
+    MT_TRY((launch_anal_f64<AnaGroups<2, 0>, 8>(a, st)));
+  }
+  {
+    AnalArgs<1, 1> a{};
+    anal_args(a, nfo - 1);
+    a.out[0] = (double2*)out->heat;
+    MT_TRY((launch_anal_f64<AnaScalar, 8>(a, st)));
+  }
+  return launch_courant_finish(n_r, mx, mx + n_r, q->delxr2, q->delxh2, dtrkc, dthkc, st);
+}
+
 // The digit-split anelastic stage runs where one CTA of its FP64 phi stage
 // holds a (theta row, level)'s buffers in shared memory.
 static bool anel_ozaki_fits(const mt_plan* p, int mag, int chem) {
@@ -1413,9 +1565,7 @@ static int nl_anel_ozaki_t(const mt_plan* p, int n_r, const mt_anel_in* in,
   }
   {
     MT_CHECK_CUDA(cudaMemsetAsync(mx, 0, 2 * n_r * sizeof(unsigned long long), st));
-    NlAnelArgs nl{};
-    nl.t = p->tab;
-    nl.n_r = n_r;
+    NlAnelArgs nl = anel_phi_args(p, n_r, MAG, q, mx);
     nl.Fs64 = Fs;
     nl.fs_m = fs_m;
     nl.fs_c = fs_c;
@@ -1425,28 +1575,6 @@ static int nl_anel_ozaki_t(const mt_plan* p, int n_r, const mt_anel_in* in,
     nl.g_h = g_h;
     nl.g_j = g_j;
     nl.g_level = W.g_level;
-    nl.r = q->r;
-    nl.or1 = q->or1;
-    nl.or2 = q->or2;
-    nl.or4 = q->or4;
-    nl.beta = q->beta;
-    nl.orho1 = q->orho1;
-    nl.orho2 = q->orho2;
-    nl.otemp1 = q->otemp1;
-    nl.visc = q->visc;
-    nl.lambda_ = q->lambda_;
-    nl.delxr2 = q->delxr2;
-    nl.delxh2 = q->delxh2;
-    nl.LFfac = q->LFfac;
-    nl.ViscHeatFac = q->ViscHeatFac;
-    nl.OhmLossFac = MAG ? q->OhmLossFac : 0.0;
-    nl.cour_mode = MAG ? q->cour_mode : 0;
-    nl.cf2 = q->courfac * q->courfac;
-    nl.af2 = q->alffac * q->alffac;
-    const double h = 0.5 * (1.0 + q->opm);
-    nl.valfac = h * h;
-    nl.vr2max = mx;
-    nl.vh2max = mx + n_r;
     MT_TRY(launch_nl_anel_f64(MAG, CHEM, nl, st));
   }
   OzAnaArgs a{};
@@ -1526,6 +1654,52 @@ int mt_nl_bouss(const mt_plan* p, int n_r, const mt_bouss_in* in, const mt_bouss
 }
 
 
+static int check_nl_anel(int n_r, const mt_anel_in* in, const mt_anel_out* out,
+                         const mt_anel_stage_params* q, const double* dtrkc,
+                         const double* dthkc) {
+  MT_REQUIRE(in && out && q && dtrkc && dthkc && n_r >= 3, MT_ERR_ARG, "bad argument");
+  MT_REQUIRE(in->w && in->dw && in->ddw && in->z && in->dz && in->s, MT_ERR_ARG,
+             "null velocity/entropy input");
+  MT_REQUIRE(!q->l_mag || (in->b && in->db && in->ddb && in->aj && in->dj), MT_ERR_ARG,
+             "null magnetic input");
+  MT_REQUIRE(!q->l_chem || in->xi, MT_ERR_ARG, "null composition input");
+  MT_REQUIRE(in->ld >= n_r && out->ld >= n_r, MT_ERR_ARG, "ld >= n_r required");
+  MT_REQUIRE(out->Advr && out->Advt && out->Advp && out->VSr && out->VSt && out->heat,
+             MT_ERR_ARG, "null output");
+  MT_REQUIRE(!q->l_mag || (out->VxBr && out->VxBt && out->VxBp), MT_ERR_ARG,
+             "null magnetic output");
+  MT_REQUIRE(!q->l_chem || (out->VXir && out->VXit), MT_ERR_ARG, "null composition output");
+  MT_REQUIRE(q->r && q->or1 && q->or2 && q->or4 && q->beta && q->orho1 && q->orho2 && q->otemp1 &&
+                 q->visc && q->lambda_ && q->delxr2 && q->delxh2,
+             MT_ERR_ARG, "null radial profile");
+  MT_REQUIRE(q->cour_mode >= 0 && q->cour_mode <= 2, MT_ERR_ARG, "bad cour_mode");
+  return MT_OK;
+}
+
+size_t mt_nl_anel_f64_workspace(const mt_plan* p, int n_r, int l_mag, int l_chem) {
+  if (!p || n_r < 3 || p->precision != MT_PREC_FP64) return 0;
+  return fourier_bytes(p, (int64_t)n_r * anel_nfi(l_mag, l_chem)) +
+         fourier_bytes(p, (int64_t)(n_r - 2) * anel_nfo(l_mag, l_chem)) +
+         2 * (size_t)n_r * sizeof(unsigned long long);
+}
+
+int mt_nl_anel_f64(const mt_plan* p, int n_r, const mt_anel_in* in, const mt_anel_out* out,
+                   const mt_anel_stage_params* q, double* dtrkc, double* dthkc, void* work,
+                   size_t work_bytes, void* stream) {
+  MT_TRY(check_plan(p));
+  MT_REQUIRE(p->precision == MT_PREC_FP64, MT_ERR_UNSUPPORTED,
+             "mt_nl_anel_f64 needs a MT_PREC_FP64 plan");
+  MT_TRY(check_nl_anel(n_r, in, out, q, dtrkc, dthkc));
+  MT_REQUIRE(work && work_bytes >= mt_nl_anel_f64_workspace(p, n_r, q->l_mag, q->l_chem),
+             MT_ERR_WORKSPACE, "workspace too small");
+  cudaStream_t st = (cudaStream_t)stream;
+  if (q->l_mag)
+    return q->l_chem ? nl_anel_f64_t<true, true>(p, n_r, in, out, q, dtrkc, dthkc, work, st)
+                     : nl_anel_f64_t<true, false>(p, n_r, in, out, q, dtrkc, dthkc, work, st);
+  return q->l_chem ? nl_anel_f64_t<false, true>(p, n_r, in, out, q, dtrkc, dthkc, work, st)
+                   : nl_anel_f64_t<false, false>(p, n_r, in, out, q, dtrkc, dthkc, work, st);
+}
+
 size_t mt_nl_anel_workspace(const mt_plan* p, int n_r, int l_mag, int l_chem) {
   if (!p || n_r < 3) return 0;
   if (p->precision == MT_PREC_SPLIT)
@@ -1546,22 +1720,7 @@ int mt_nl_anel(const mt_plan* p, int n_r, const mt_anel_in* in, const mt_anel_ou
              MT_ERR_UNSUPPORTED,
              "n_phi too long for the digit-split anelastic stage's phi buffers (compose the "
              "drop-in transforms and mt_get_nl_anel instead)");
-  MT_REQUIRE(in && out && q && dtrkc && dthkc && n_r >= 3, MT_ERR_ARG, "bad argument");
-  MT_REQUIRE(in->w && in->dw && in->ddw && in->z && in->dz && in->s, MT_ERR_ARG,
-             "null velocity/entropy input");
-  MT_REQUIRE(!q->l_mag || (in->b && in->db && in->ddb && in->aj && in->dj), MT_ERR_ARG,
-             "null magnetic input");
-  MT_REQUIRE(!q->l_chem || in->xi, MT_ERR_ARG, "null composition input");
-  MT_REQUIRE(in->ld >= n_r && out->ld >= n_r, MT_ERR_ARG, "ld >= n_r required");
-  MT_REQUIRE(out->Advr && out->Advt && out->Advp && out->VSr && out->VSt && out->heat,
-             MT_ERR_ARG, "null output");
-  MT_REQUIRE(!q->l_mag || (out->VxBr && out->VxBt && out->VxBp), MT_ERR_ARG,
-             "null magnetic output");
-  MT_REQUIRE(!q->l_chem || (out->VXir && out->VXit), MT_ERR_ARG, "null composition output");
-  MT_REQUIRE(q->r && q->or1 && q->or2 && q->or4 && q->beta && q->orho1 && q->orho2 && q->otemp1 &&
-                 q->visc && q->lambda_ && q->delxr2 && q->delxh2,
-             MT_ERR_ARG, "null radial profile");
-  MT_REQUIRE(q->cour_mode >= 0 && q->cour_mode <= 2, MT_ERR_ARG, "bad cour_mode");
+  MT_TRY(check_nl_anel(n_r, in, out, q, dtrkc, dthkc));
   MT_REQUIRE(work && work_bytes >= mt_nl_anel_workspace(p, n_r, q->l_mag, q->l_chem),
              MT_ERR_WORKSPACE, "workspace too small");
   cudaStream_t st = (cudaStream_t)stream;

@@ -3,7 +3,8 @@
 // A synthesis operation contracts, per order m, the tables P and
 // dP = sin(theta) dP/dtheta (rows l, columns northern theta) with NX complex
 // input terms per column (radial level / batch entry).  Products are (table,
-// term) pairs; the epilogue turns products into NO output fields.
+// term) pairs; the epilogue turns products into NO output fields, output f
+// being grid field field(f) of the column.
 //
 // Equatorial folding (reference magic_torch/sht.py:120-149): rows with
 // (l - m) even (E) and odd (O) are summed separately; then
@@ -50,6 +51,7 @@ __device__ __forceinline__ dcx scale(dcx a, double s) { return {s * a.x, s * a.y
 
 struct SynScalar {
   static constexpr int NX = 1, NP = 1, NO = 1, NT = 1;
+  __host__ __device__ static constexpr int field(int f) { return f; }
   __host__ __device__ static constexpr int table(int) { return kP; }
   __host__ __device__ static constexpr int term(int) { return 0; }
   __device__ static void combine(const dcx* h, double, dcx* o) { o[0] = h[0]; }
@@ -57,6 +59,7 @@ struct SynScalar {
 
 struct SynGrad {  // (dP X, i m P X) -> (d/dtheta, 1/sin d/dphi), sin-weighted
   static constexpr int NX = 1, NP = 2, NO = 2, NT = 2;
+  __host__ __device__ static constexpr int field(int f) { return f; }
   __host__ __device__ static constexpr int table(int p) { return p == 0 ? kDP : kP; }
   __host__ __device__ static constexpr int term(int) { return 0; }
   __device__ static void combine(const dcx* h, double m, dcx* o) {
@@ -79,6 +82,7 @@ __device__ __forceinline__ void torpol_combine(const dcx* h, double m, dcx* o) {
 
 struct SynTorpol {
   static constexpr int NX = 3, NP = 5, NO = 3, NT = 2;
+  __host__ __device__ static constexpr int field(int f) { return f; }
   __host__ __device__ static constexpr int table(int p) { return torpol_table(p); }
   __host__ __device__ static constexpr int term(int p) { return torpol_term(p); }
   __device__ static void combine(const dcx* h, double m, dcx* o) { torpol_combine(h, m, o); }
@@ -92,6 +96,7 @@ struct SynGroups {
   static constexpr int NX = 3 * G + NS;
   static constexpr int NP = 5 * G + NS;
   static constexpr int NO = NX, NT = 2;
+  __host__ __device__ static constexpr int field(int f) { return f; }
   __host__ __device__ static constexpr int table(int p) {
     return p < 5 * G ? torpol_table(p % 5) : kP;
   }
@@ -104,6 +109,35 @@ struct SynGroups {
 #pragma unroll
     for (int si = 0; si < NS; ++si) o[3 * G + si] = h[5 * G + si];
   }
+};
+
+// The anelastic stage's grid fields (order of nl_point.cuh) in two operations.
+// Velocity and its horizontal derivatives, terms l(l+1) w, dw, z, l(l+1) z: the
+// phi derivatives of v_theta and v_phi are i m times their sums, so seven
+// products give eight fields (pol_to_grad_spat, torpol_to_dphspat without its
+// 1/sin^2, pol_to_curlr_spat: magic_torch/sht.py:687-743).
+struct SynAnelVel {
+  static constexpr int NX = 4, NP = 7, NO = 8, NT = 2;
+  __host__ __device__ static constexpr int field(int f) { return f < 3 ? f : f + 3; }
+  __host__ __device__ static constexpr int table(int p) { return p >= 3 && p < 6 ? kDP : kP; }
+  __host__ __device__ static constexpr int term(int p) {
+    return p < 3 ? p : p == 3 ? 1 : p == 4 ? 2 : p == 5 ? 0 : 3;
+  }
+  __device__ static void combine(const dcx* h, double m, dcx* o) {
+    torpol_combine(h, m, o);
+    o[3] = h[5];
+    o[4] = times_im(h[0], m);
+    o[5] = times_im(o[1], m);
+    o[6] = times_im(o[2], m);
+    o[7] = h[6];
+  }
+};
+
+// Radial derivatives of the velocity (terms l(l+1) dw, ddw, dz) and the scalars
+// s [, xi].
+template <int NS>
+struct SynAnelDr : SynGroups<1, NS> {
+  __host__ __device__ static constexpr int field(int f) { return f < 3 ? 3 + f : 8 + f; }
 };
 
 // ----------------------------------------------------------------- analysis
@@ -194,6 +228,7 @@ struct AnalArgs {
   double2* out[NO];  // (lm_max, ld) arrays
   int64_t ld;
   int out_col0;      // output column = out_col0 + c
+  int zero_ends;     // also zero the output columns on either side
 };
 
 }  // namespace mt

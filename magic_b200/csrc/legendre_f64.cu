@@ -188,8 +188,8 @@ __global__ void __launch_bounds__(256, 2) k_synth_f64(SynthArgs<OP::NX> a) {
     double2* FS = FN + a.f_row;
 #pragma unroll
     for (int f = 0; f < NO; ++f) {
-      FN[f * a.col_f] = make_double2(oN[f].x, oN[f].y);
-      FS[f * a.col_f] = make_double2(oS[f].x, oS[f].y);
+      FN[OP::field(f) * a.col_f] = make_double2(oN[f].x, oN[f].y);
+      FS[OP::field(f) * a.col_f] = make_double2(oS[f].x, oS[f].y);
     }
   }
 }
@@ -330,7 +330,11 @@ __global__ void __launch_bounds__(256, 2) k_anal_f64(AnalArgs<OP::NX, OP::NO> a)
     const int64_t off = (int64_t)(ls + k) * a.ld + a.out_col0 + col;
 #pragma unroll
     for (int f = 0; f < NO; ++f)
-      if (a.out[f]) a.out[f][off] = make_double2(o[f].x, o[f].y);
+      if (a.out[f]) {
+        a.out[f][off] = make_double2(o[f].x, o[f].y);
+        if (a.zero_ends && col == 0) a.out[f][off - 1] = make_double2(0.0, 0.0);
+        if (a.zero_ends && col == a.ncols - 1) a.out[f][off + 1] = make_double2(0.0, 0.0);
+      }
   }
 }
 
@@ -368,6 +372,9 @@ template int launch_synth_f64<SynTorpol, 8>(const SynthArgs<3>&, cudaStream_t);
 template int launch_synth_f64<SynGroups<2, 0>, 8>(const SynthArgs<6>&, cudaStream_t);
 template int launch_synth_f64<SynGroups<2, 1>, 8>(const SynthArgs<7>&, cudaStream_t);
 template int launch_synth_f64<SynGroups<2, 2>, 8>(const SynthArgs<8>&, cudaStream_t);
+template int launch_synth_f64<SynAnelVel, 8>(const SynthArgs<4>&, cudaStream_t);
+template int launch_synth_f64<SynAnelDr<1>, 8>(const SynthArgs<4>&, cudaStream_t);
+template int launch_synth_f64<SynAnelDr<2>, 8>(const SynthArgs<5>&, cudaStream_t);
 template int launch_anal_f64<AnaScalar, 8>(const AnalArgs<1, 1>&, cudaStream_t);
 template int launch_anal_f64<AnaSphtor, 8>(const AnalArgs<2, 2>&, cudaStream_t);
 template int launch_anal_f64<AnaGroups<1, 2>, 8>(const AnalArgs<6, 5>&, cudaStream_t);

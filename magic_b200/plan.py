@@ -444,99 +444,18 @@ class Plan:
                                    D1._h if D1 is not None else None, self._stream()))
         return out
 
-    def _nl_anel_composed(self, fields, prof, LFfac, ViscHeatFac, OhmLossFac, courfac, alffac,
-                          opm, l_mag, l_chem, damp, out):
-        """FP64 plans: the anelastic nonlinear stage composed, as the reference's
-        radial_loop_anel composes it (step_time.py:1233-1474), from the FP64 transform
-        kernels, mt_get_nl_anel and mt_courant, with the grids in device memory:
-        s, xi and the magnetic field on every level; velocity, its radial, theta and
-        phi derivatives and cvr on the bulk levels (zero on both boundaries); forward
-        transforms of the bulk levels; Courant steps from the zero-boundary velocity."""
-        n_r = fields["w"].shape[1]
-        for k in ["w", "dw", "ddw", "z", "dz", "s"] + (["b", "db", "ddb", "aj", "dj"] if l_mag
-                                                       else []) + (["xi"] if l_chem else []):
-            x = fields[k]
-            if x.shape != (self.lm_max, n_r) or x.dtype != _CD or x.device != self.device:
-                raise ValueError(f"fields[{k}]: expected ({self.lm_max}, {n_r}) complex128")
-        if n_r < 3:
-            raise MagicError("nl_anel needs n_r >= 3")
-        shape = (n_r, self.n_theta_max, self.n_phi_max)
-        zeros = lambda: torch.zeros(shape, dtype=_RD, device=self.device)
-        d = self.dLh.unsqueeze(1)
-        o2 = self._prof(prof["or2"], n_r).unsqueeze(0)
-        sc = self.scal_to_spat(fields["s"])
-        xic = self.scal_to_spat(fields["xi"]) if l_chem else zeros()
-        if l_mag:
-            br, bt, bp = self.torpol_to_spat(d * fields["b"], fields["db"], fields["aj"])
-            cbr, cbt, cbp = self.torpol_to_spat(d * fields["aj"], fields["dj"],
-                                                o2 * d * fields["b"] - fields["ddb"])
-        else:
-            br, bt, bp, cbr, cbt, cbp = (zeros() for _ in range(6))
-        bk = slice(1, n_r - 1)
-        wb, dwb, ddwb, zb, dzb = (fields[k][:, bk] for k in ("w", "dw", "ddw", "z", "dz"))
-
-        def bulk(*grids):
-            res = []
-            for x in grids:
-                a = zeros()
-                a[bk] = x
-                res.append(a)
-            return res
-
-        vr, vt, vp = bulk(*self.torpol_to_spat(d * wb, dwb, zb))
-        dvrdr, dvtdr, dvpdr = bulk(*self.torpol_to_spat(d * dwb, ddwb, dzb))
-        (cvr,) = bulk(self.scal_to_spat(d * zb))
-        dvrdt, dvrdp = bulk(*self.pol_to_grad_spat(wb))
-        ph = self.dPhi.unsqueeze(1)
-        _, gt, gp = self.torpol_to_spat(torch.zeros_like(dwb), ph * dwb, ph * zb)
-        ost = self.O_sin_theta_E2_grid.unsqueeze(1)
-        dvtdp, dvpdp = bulk(gt * ost, gp * ost)
-        nl = self.get_nl_anel([vr, vt, vp, dvrdr, dvtdr, dvpdr, dvrdt, dvrdp, dvtdp, dvpdp, cvr,
-                               sc, xic, br, bt, bp, cbr, cbt, cbp], prof, LFfac, ViscHeatFac,
-                              OhmLossFac, l_mag)
-        Advr, Advt, Advp, VSr, VSt, VSp, VxBr, VxBt, VxBp, VXir, VXit, VXip, heat = nl
-        onames = ["Advr", "Advt", "Advp", "VSr", "VSt"] + (["VxBr", "VxBt", "VxBp"] if l_mag
-                                                           else []) + \
-            (["VXir", "VXit"] if l_chem else []) + ["heat"]
-        if out is None:
-            out = {k: torch.zeros(self.lm_max, n_r, dtype=_CD, device=self.device) for k in onames}
-
-        def put(name, x):
-            out[name][:, 0] = 0.0
-            out[name][:, -1] = 0.0
-            out[name][:, bk] = x
-
-        put("Advr", self.scal_to_SH(Advr[bk]))
-        put("VSr", self.scal_to_SH(VSr[bk]))
-        S, T = self.spat_to_sphertor(Advt[bk], Advp[bk])
-        put("Advt", S)
-        put("Advp", T)
-        put("VSt", self.spat_to_sphertor(VSt[bk], VSp[bk])[0])
-        if l_mag:
-            put("VxBr", self.scal_to_SH(VxBr[bk]))
-            S, T = self.spat_to_sphertor(VxBt[bk], VxBp[bk])
-            put("VxBt", S)
-            put("VxBp", T)
-        if l_chem:
-            put("VXir", self.scal_to_SH(VXir[bk]))
-            put("VXit", self.spat_to_sphertor(VXit[bk], VXip[bk])[0])
-        put("heat", self.scal_to_SH(heat[bk]))
-        dtr, dth = self.courant(vr, vt, vp, br if l_mag else None, bt, bp, prof, courfac, alffac,
-                                LFfac, opm, damp=damp)
-        return out, dtr, dth
-
     def nl_anel_workspace(self, n_r, l_mag=True, l_chem=False):
-        return _lib.lib().mt_nl_anel_workspace(self._h, int(n_r), int(l_mag), int(l_chem))
+        L = _lib.lib()
+        size = L.mt_nl_anel_f64_workspace if self.precision == "fp64" else L.mt_nl_anel_workspace
+        return size(self._h, int(n_r), int(l_mag), int(l_chem))
 
     def nl_anel(self, fields, prof, LFfac, ViscHeatFac, OhmLossFac, courfac, alffac, opm,
                 l_mag=True, l_chem=False, damp=True, out=None, work=None):
         """Anelastic nonlinear stage (magic_torch/step_time.py:1215-1475: transforms,
-        get_nl_anel with viscous and Ohmic heating, forward transforms, CFL): fused into
-        the tcgen05 pack/GEMM and FP32 phi kernels on split-precision plans, into the
-        int8 digit-plane GEMMs and an FP64 phi kernel on digit-split (ozaki) plans, and
-        composed from the FP64 kernels on FP64 plans (and on a digit-split plan whose
-        phi rows would not fit one CTA's shared memory, which no plan within the
-        library's n_phi limit reaches).
+        get_nl_anel with viscous and Ohmic heating, forward transforms, CFL), fused: the
+        tcgen05 pack/GEMM and FP32 phi kernels on split-precision plans, the int8
+        digit-plane GEMMs and an FP64 phi kernel on digit-split (ozaki) plans, the FP64
+        contractions and the same phi kernel on FP64 plans.
 
         ``fields``: dict of spectral (lm_max, n_r) complex128 arrays w, dw, ddw, z, dz, s
         (+ b, db, ddb, aj, dj if l_mag, xi if l_chem).  ``prof``: r, or1, or2, or4, beta,
@@ -547,12 +466,6 @@ class Plan:
         w = fields["w"]
         n_r = w.shape[1]
         L = _lib.lib()
-        need = L.mt_nl_anel_workspace(self._h, n_r, int(l_mag), int(l_chem)) if n_r >= 3 else 0
-        if self.precision == "fp64" or (self.precision == "ozaki" and need == 0):
-            return self._nl_anel_composed(fields, prof, LFfac, ViscHeatFac, OhmLossFac, courfac,
-                                          alffac, opm, l_mag, l_chem, damp, out)
-        if need == 0:
-            raise MagicError("nl_anel needs n_r >= 3")
         names = ["w", "dw", "ddw", "z", "dz", "s"] + (["b", "db", "ddb", "aj", "dj"] if l_mag
                                                        else []) + (["xi"] if l_chem else [])
         ins = {}
@@ -560,12 +473,30 @@ class Plan:
             x = fields[k]
             if x.shape != (self.lm_max, n_r) or x.dtype != _CD or x.device != self.device:
                 raise ValueError(f"fields[{k}]: expected ({self.lm_max}, {n_r}) complex128")
-            ins[k] = x.contiguous()
+            ins[k] = x.resolve_conj().contiguous()
+        need = self.nl_anel_workspace(n_r, l_mag, l_chem) if n_r >= 3 else 0
+        if need == 0:
+            raise MagicError("nl_anel needs n_r >= 3")
         onames = ["Advr", "Advt", "Advp", "VSr", "VSt"] + (["VxBr", "VxBt", "VxBp"] if l_mag
                                                            else []) + \
             (["VXir", "VXit"] if l_chem else []) + ["heat"]
         if out is None:
             out = {k: torch.zeros(self.lm_max, n_r, dtype=_CD, device=self.device) for k in onames}
+        # FP64 plans take outputs of any layout and type: what the kernels cannot write
+        # (complex128 rows of unit stride, one row stride for all) goes through a copy
+        given = out
+        if self.precision == "fp64":
+            o0 = out[onames[0]]
+            fits = all(x.shape == (self.lm_max, n_r) and x.dtype == _CD
+                       and x.device == self.device and x.stride(1) == 1
+                       and x.stride(0) == o0.stride(0) >= n_r and not x.is_conj()
+                       for x in (out[k] for k in onames))
+            if not fits:
+                out = {k: torch.empty(self.lm_max, n_r, dtype=_CD, device=self.device)
+                       for k in onames}
+            if work is not None and (work.device != self.device or not work.is_contiguous()
+                                     or work.dtype != torch.uint8 or work.data_ptr() % 16):
+                work = None
         pnames = ("r", "or1", "or2", "or4", "beta", "orho1", "orho2", "otemp1", "visc",
                   "lambda_", "delxr2", "delxh2")
         keep = {k: self._prof(prof[k], n_r) for k in pnames}
@@ -583,7 +514,13 @@ class Plan:
         dth = torch.empty_like(dtr)
         if work is None or work.numel() < need:
             work = self._work(need)
-        check(L.mt_nl_anel(self._h, n_r, C.byref(ai), C.byref(ao), C.byref(ap), _ptr(dtr),
-                           _ptr(dth), _ptr(work), work.numel(), self._stream()))
+        run = L.mt_nl_anel_f64 if self.precision == "fp64" else L.mt_nl_anel
+        check(run(self._h, n_r, C.byref(ai), C.byref(ao), C.byref(ap), _ptr(dtr), _ptr(dth),
+                  _ptr(work), work.numel(), self._stream()))
         self._watch(work, "nl_anel", fused=True)
-        return out, dtr, dth
+        if out is not given:
+            for k in onames:
+                given[k][:, 0] = 0.0
+                given[k][:, -1] = 0.0
+                given[k][:, 1:n_r - 1] = out[k][:, 1:-1]
+        return given, dtr, dth

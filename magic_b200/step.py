@@ -485,12 +485,9 @@ class AnelasticStep(BoussinesqStep):
 
     @property
     def work(self):
-        """Workspace of the fused (split or digit-split) anelastic stage; FP64 plans
-        compose the stage from the FP64 kernels and need none (the plan reports 0
-        where the digit-split stage composes too)."""
+        """Workspace of the fused anelastic stage."""
         if self._work is None:
-            n = self.plan.nl_anel_workspace(self.n_r, self.l_mag, False) \
-                if self.plan.precision in ("split", "ozaki") else 0
+            n = self.plan.nl_anel_workspace(self.n_r, self.l_mag, False)
             self._work = torch.empty(max(int(n), 1), dtype=torch.uint8, device=self.device)
         return self._work
 
