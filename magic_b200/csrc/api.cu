@@ -316,7 +316,7 @@ int mt_scal_to_spat(const mt_plan* p, const double* Slm, int64_t ld, int B, doub
   double2* F = (double2*)work;
   SynthArgs<1> s{};
   s.t = p->tab;
-  s.src[0] = {(const double2*)Slm, nullptr, kRaw};
+  s.src[0] = (const double2*)Slm;
   s.ld = ld;
   s.ncols = B;
   s.F = F;
@@ -398,7 +398,7 @@ int mt_scal_to_grad_spat(const mt_plan* p, const double* Slm, int64_t ld, int B,
   double2* F = (double2*)work;
   SynthArgs<1> s{};
   s.t = p->tab;
-  s.src[0] = {(const double2*)Slm, nullptr, scale_dlh ? kDlh : kRaw};
+  s.src[0] = (const double2*)Slm;
   s.ld = ld;
   s.ncols = B;
   s.F = F;
@@ -406,7 +406,8 @@ int mt_scal_to_grad_spat(const mt_plan* p, const double* Slm, int64_t ld, int B,
   s.f_m = (int64_t)p->n_theta * s.f_row;
   s.col_f = B;
   s.col_c = 1;
-  MT_TRY((launch_synth_f64<SynGrad, 16>(s, st)));
+  if (scale_dlh) MT_TRY((launch_synth_f64<SynGrad<true>, 16>(s, st)));
+  else MT_TRY((launch_synth_f64<SynGrad<false>, 16>(s, st)));
   ToGridArgs g{};
   g.t = p->tab;
   g.F = F;
@@ -437,9 +438,9 @@ int mt_torpol_to_spat(const mt_plan* p, const double* Q, const double* S, const 
   double2* F = (double2*)work;
   SynthArgs<3> s{};
   s.t = p->tab;
-  s.src[0] = {(const double2*)Q, nullptr, kRaw};
-  s.src[1] = {(const double2*)S, nullptr, kRaw};
-  s.src[2] = {(const double2*)T, nullptr, kRaw};
+  s.src[0] = (const double2*)Q;
+  s.src[1] = (const double2*)S;
+  s.src[2] = (const double2*)T;
   s.ld = ld;
   s.ncols = B;
   s.F = F;
@@ -447,7 +448,7 @@ int mt_torpol_to_spat(const mt_plan* p, const double* Q, const double* S, const 
   s.f_m = (int64_t)p->n_theta * s.f_row;
   s.col_f = B;
   s.col_c = 1;
-  MT_TRY((launch_synth_f64<SynTorpol, 8>(s, st)));
+  MT_TRY((launch_synth_f64<SynTorpol, 4>(s, st)));
   ToGridArgs g{};
   g.t = p->tab;
   g.F = F;
@@ -675,12 +676,13 @@ static int nl_bouss_t(const mt_plan* p, int n_r, const mt_bouss_in* in, const mt
   if ((parts & 1) && MAG) {
     SynthArgs<6> s{};
     s.t = p->tab;
-    s.src[0] = {c(in->b), nullptr, kDlh};
-    s.src[1] = {c(in->db), nullptr, kRaw};
-    s.src[2] = {c(in->aj), nullptr, kRaw};
-    s.src[3] = {c(in->aj), nullptr, kDlh};
-    s.src[4] = {c(in->dj), nullptr, kRaw};
-    s.src[5] = {c(in->b), c(in->ddb), kCurlT};
+    s.src[0] = c(in->b);
+    s.src[1] = c(in->db);
+    s.src[2] = c(in->aj);
+    s.src[3] = c(in->aj);
+    s.src[4] = c(in->dj);
+    s.src[5] = c(in->b);
+    s.curl_b = c(in->ddb);
     s.ld = in->ld;
     s.ncols = n_r;
     s.or2 = q->or2;
@@ -689,20 +691,21 @@ static int nl_bouss_t(const mt_plan* p, int n_r, const mt_bouss_in* in, const mt
     s.f_m = f_m;
     s.col_f = 1;
     s.col_c = nfi;
-    MT_TRY((launch_synth_f64<SynGroups<2, 0>, 8>(s, st)));
+    MT_TRY((launch_synth_f64<SynGroups<2, 0>, 4>(s, st)));
   }
   if (parts & 1) {
     using SO = SynGroups<2, CHEM ? 2 : 1>;
     SynthArgs<SO::NX> s{};
     s.t = p->tab;
-    s.src[0] = {c(in->w), nullptr, kDlh};
-    s.src[1] = {c(in->dw), nullptr, kRaw};
-    s.src[2] = {c(in->z), nullptr, kRaw};
-    s.src[3] = {c(in->z), nullptr, kDlh};
-    s.src[4] = {c(in->dz), nullptr, kRaw};
-    s.src[5] = {c(in->w), c(in->ddw), kCurlT};
-    s.src[6] = {c(in->s), nullptr, kRaw};
-    if (CHEM) s.src[SO::NX - 1] = {c(in->xi), nullptr, kRaw};
+    s.src[0] = c(in->w);
+    s.src[1] = c(in->dw);
+    s.src[2] = c(in->z);
+    s.src[3] = c(in->z);
+    s.src[4] = c(in->dz);
+    s.src[5] = c(in->w);
+    s.curl_b = c(in->ddw);
+    s.src[6] = c(in->s);
+    if (CHEM) s.src[SO::NX - 1] = c(in->xi);
     s.ld = in->ld;
     s.ncols = n_r;
     s.or2 = q->or2;
@@ -711,7 +714,7 @@ static int nl_bouss_t(const mt_plan* p, int n_r, const mt_bouss_in* in, const mt
     s.f_m = f_m;
     s.col_f = 1;
     s.col_c = nfi;
-    MT_TRY((launch_synth_f64<SO, 8>(s, st)));
+    MT_TRY((launch_synth_f64<SO, 4>(s, st)));
   }
 
   NlBoussArgs nl{};
@@ -1431,33 +1434,34 @@ static int nl_anel_f64_t(const mt_plan* p, int n_r, const mt_anel_in* in, const 
   {
     SynthArgs<4> s{};
     synth_args(s, 0);
-    s.src[0] = {c(in->w), nullptr, kDlh};
-    s.src[1] = {c(in->dw), nullptr, kRaw};
-    s.src[2] = {c(in->z), nullptr, kRaw};
-    s.src[3] = {c(in->z), nullptr, kDlh};
-    MT_TRY((launch_synth_f64<SynAnelVel, 8>(s, st)));
+    s.src[0] = c(in->w);
+    s.src[1] = c(in->dw);
+    s.src[2] = c(in->z);
+    s.src[3] = c(in->z);
+    MT_TRY((launch_synth_f64<SynAnelVel, 4>(s, st)));
   }
   {
     using SO = SynAnelDr<CHEM ? 2 : 1>;
     SynthArgs<SO::NX> s{};
     synth_args(s, 0);
-    s.src[0] = {c(in->dw), nullptr, kDlh};
-    s.src[1] = {c(in->ddw), nullptr, kRaw};
-    s.src[2] = {c(in->dz), nullptr, kRaw};
-    s.src[3] = {c(in->s), nullptr, kRaw};
-    if (CHEM) s.src[SO::NX - 1] = {c(in->xi), nullptr, kRaw};
-    MT_TRY((launch_synth_f64<SO, 8>(s, st)));
+    s.src[0] = c(in->dw);
+    s.src[1] = c(in->ddw);
+    s.src[2] = c(in->dz);
+    s.src[3] = c(in->s);
+    if (CHEM) s.src[SO::NX - 1] = c(in->xi);
+    MT_TRY((launch_synth_f64<SO, 4>(s, st)));
   }
   if (MAG) {
     SynthArgs<6> s{};
     synth_args(s, 12 + (CHEM ? 1 : 0));
-    s.src[0] = {c(in->b), nullptr, kDlh};
-    s.src[1] = {c(in->db), nullptr, kRaw};
-    s.src[2] = {c(in->aj), nullptr, kRaw};
-    s.src[3] = {c(in->aj), nullptr, kDlh};
-    s.src[4] = {c(in->dj), nullptr, kRaw};
-    s.src[5] = {c(in->b), c(in->ddb), kCurlT};
-    MT_TRY((launch_synth_f64<SynGroups<2, 0>, 8>(s, st)));
+    s.src[0] = c(in->b);
+    s.src[1] = c(in->db);
+    s.src[2] = c(in->aj);
+    s.src[3] = c(in->aj);
+    s.src[4] = c(in->dj);
+    s.src[5] = c(in->b);
+    s.curl_b = c(in->ddb);
+    MT_TRY((launch_synth_f64<SynGroups<2, 0>, 4>(s, st)));
   }
   MT_CHECK_CUDA(cudaMemsetAsync(mx, 0, 2 * n_r * sizeof(unsigned long long), st));
   NlAnelArgs nl = anel_phi_args(p, n_r, MAG, q, mx);

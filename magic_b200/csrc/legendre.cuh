@@ -23,19 +23,11 @@ namespace mt {
 
 enum Table : int { kP = 0, kDP = 1 };
 
-// Term recipes applied while loading spectral inputs (radial-loop assembly,
-// magic_torch/step_time.py:980-1013).
+// Term recipes (radial-loop assembly, magic_torch/step_time.py:980-1013).
 enum Recipe : int {
-  kRaw = 0,    // X = A
-  kDlh = 1,    // X = l(l+1) A
-  kCurlT = 2,  // X = or2[col] l(l+1) A - B
-  kZero = 3    // X = 0
-};
-
-struct TermSrc {
-  const double2* a;
-  const double2* b;
-  int recipe;
+  kRaw = 0,   // X = A
+  kDlh = 1,   // X = l(l+1) A
+  kCurlT = 2  // X = or2[col] l(l+1) A - B
 };
 
 struct dcx {
@@ -52,14 +44,17 @@ __device__ __forceinline__ dcx scale(dcx a, double s) { return {s * a.x, s * a.y
 struct SynScalar {
   static constexpr int NX = 1, NP = 1, NO = 1, NT = 1;
   __host__ __device__ static constexpr int field(int f) { return f; }
+  __host__ __device__ static constexpr int recipe(int) { return kRaw; }
   __host__ __device__ static constexpr int table(int) { return kP; }
   __host__ __device__ static constexpr int term(int) { return 0; }
   __device__ static void combine(const dcx* h, double, dcx* o) { o[0] = h[0]; }
 };
 
+template <bool DLH>  // of l(l+1) X
 struct SynGrad {  // (dP X, i m P X) -> (d/dtheta, 1/sin d/dphi), sin-weighted
   static constexpr int NX = 1, NP = 2, NO = 2, NT = 2;
   __host__ __device__ static constexpr int field(int f) { return f; }
+  __host__ __device__ static constexpr int recipe(int) { return DLH ? kDlh : kRaw; }
   __host__ __device__ static constexpr int table(int p) { return p == 0 ? kDP : kP; }
   __host__ __device__ static constexpr int term(int) { return 0; }
   __device__ static void combine(const dcx* h, double m, dcx* o) {
@@ -83,6 +78,7 @@ __device__ __forceinline__ void torpol_combine(const dcx* h, double m, dcx* o) {
 struct SynTorpol {
   static constexpr int NX = 3, NP = 5, NO = 3, NT = 2;
   __host__ __device__ static constexpr int field(int f) { return f; }
+  __host__ __device__ static constexpr int recipe(int) { return kRaw; }
   __host__ __device__ static constexpr int table(int p) { return torpol_table(p); }
   __host__ __device__ static constexpr int term(int p) { return torpol_term(p); }
   __device__ static void combine(const dcx* h, double m, dcx* o) { torpol_combine(h, m, o); }
@@ -97,6 +93,10 @@ struct SynGroups {
   static constexpr int NP = 5 * G + NS;
   static constexpr int NO = NX, NT = 2;
   __host__ __device__ static constexpr int field(int f) { return f; }
+  // Q of a group is l(l+1) times its potential; the second group is a curl
+  __host__ __device__ static constexpr int recipe(int x) {
+    return x == 5 && G == 2 ? kCurlT : x < 3 * G && x % 3 == 0 ? kDlh : kRaw;
+  }
   __host__ __device__ static constexpr int table(int p) {
     return p < 5 * G ? torpol_table(p % 5) : kP;
   }
@@ -119,6 +119,7 @@ struct SynGroups {
 struct SynAnelVel {
   static constexpr int NX = 4, NP = 7, NO = 8, NT = 2;
   __host__ __device__ static constexpr int field(int f) { return f < 3 ? f : f + 3; }
+  __host__ __device__ static constexpr int recipe(int x) { return x % 3 ? kRaw : kDlh; }
   __host__ __device__ static constexpr int table(int p) { return p >= 3 && p < 6 ? kDP : kP; }
   __host__ __device__ static constexpr int term(int p) {
     return p < 3 ? p : p == 3 ? 1 : p == 4 ? 2 : p == 5 ? 0 : 3;
@@ -209,7 +210,8 @@ struct AnaGroups {
 template <int NX>
 struct SynthArgs {
   Tables t;
-  TermSrc src[NX];
+  const double2* src[NX];
+  const double2* curl_b;  // B of the term with recipe kCurlT
   int64_t ld;         // row stride of the spectral sources (complex elements)
   int ncols;          // columns (levels / batch entries)
   const double* or2;  // (ncols) for kCurlT
