@@ -922,8 +922,16 @@ inline size_t oz_ana_pack_smem(int nhs, int rb) {
   return (size_t)2 * nhs * rb * 8 + (size_t)2 * (kOzPackThreads + rb) * 8;
 }
 
+// The load and digit passes of one CTA do not overlap, and two or three CTAs an SM
+// leave HBM idle while they split digits; so a CTA also prefetches into L2 the rows
+// of the one that follows two waves later.  Stage at l_max 255 on 97 levels: 5.546
+// -> 5.43 ms, anelastic at l_max 383 on 129 levels 15.0 -> 14.83, at l_max 127 on 65
+// levels 1.033 -> 0.998 ms with the third CTA that 80 registers allow where shared
+// memory does.
+constexpr int kOzPackAhead = 2 * 148;
+
 template <int RB>
-__global__ void __launch_bounds__(kOzPackThreads, 2) k_oz_ana_pack(OzAnaArgs a) {
+__global__ void __launch_bounds__(kOzPackThreads, 3) k_oz_ana_pack(OzAnaArgs a) {
   extern __shared__ __align__(16) double stg[];  // [hemisphere][theta pair][row]
   constexpr int NG = kOzPackThreads / RB;        // theta-pair groups of the load pass
   const Tables& t = a.t;
@@ -970,6 +978,24 @@ __global__ void __launch_bounds__(kOzPackThreads, 2) k_oz_ana_pack(OzAnaArgs a) 
     }
     red[g * RB + rr] = m0;
     red[(NG + g) * RB + rr] = m1;
+  }
+  {
+    // the block two waves of SMs on: its rows into L2 while this one computes
+    const int64_t nb = (int64_t)blockIdx.y * gridDim.x + blockIdx.x + kOzPackAhead;
+    if (nb < (int64_t)gridDim.x * gridDim.y) {
+      const int bx = (int)(nb % gridDim.x), mc2 = (int)(nb / gridDim.x);
+      constexpr int NL = (RB * 8 + 127) / 128;  // lines of a (theta pair, hemisphere)
+      const int lv2 = (bx / (kOzRows / RB)) * a.lev_tile;
+      const int R2 = (bx % (kOzRows / RB)) * RB;
+      for (int e = tid; e < 2 * nhs * NL; e += kOzPackThreads) {
+        const int R = R2 + 16 * (e % NL), h = e / NL / nhs, j = e / NL - h * nhs;
+        const int lv = R / a.cols;
+        if (lv < a.lev_tile && lv2 + lv < a.n_lev)
+          asm volatile("prefetch.global.L2 [%0];\n" ::"l"(
+              a.G + (int64_t)mc2 * a.g_m + h * a.g_h + (int64_t)j * a.g_j +
+              (int64_t)(lv2 + lv) * a.g_level + (R - lv * a.cols)));
+      }
+    }
   }
   __syncthreads();
   if (tid < 2 * RB) {
