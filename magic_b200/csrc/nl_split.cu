@@ -222,6 +222,23 @@ __global__ void __maxnreg__(72)
   const int tid = threadIdx.x, hw = tid >> 4, lane = tid & 15;
   const unsigned mask = 0xFFFFu << (16 * (hw & 1));
   hw_twiddles_to_smem<Q>(tw2, tw3, twN, t.twiddle, tid, T);
+  // The rows of the CTA that takes this one's place, four a SM later, into L2 (asked
+  // for by one of the two CTAs that read a theta pair): the load phase waited for HBM
+  // at 9 % of its bandwidth.  Stage at l_max 85 on 49 levels 257 -> 254 us, at l_max
+  // 127 on 65 levels 609 -> 599.
+  if ((row & 1) == 0) {
+    constexpr int kAhead = 4 * 148;
+    const int id = r * gridDim.x + row + kAhead, r2 = id / gridDim.x, row2 = id - r2 * gridDim.x;
+    if (r2 < a.n_r) {
+      const float* x = a.Fs + (int64_t)(row2 >> 1) * a.fs_j + (int64_t)r2 * 2 * NFI;
+      for (int e = tid; e < 2 * M; e += T) {
+        const float* p = x + (int64_t)(e >> 1) * a.fs_m + (e & 1) * a.fs_c;
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+        if ((reinterpret_cast<uintptr_t>(p) & 127) + 8 * NFI > 128)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(p + 2 * NFI - 1));
+      }
+    }
+  }
   // Fourier rows: element e = (k, f) of the NFI (sym, asym) pairs of
   // wavenumber k (consecutive threads read consecutive fields of one k);
   // wavenumbers k >= n_m are zero.
