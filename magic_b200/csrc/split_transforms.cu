@@ -9,8 +9,8 @@
 // by 1/N and by the row's quadrature weight (2 pi w, or 2 pi w / sin^2 for
 // vector components), written as north/south Fourier rows for the analysis
 // packing kernel.  One CTA = (theta row, up to kPhiRows rows); the FFT is the
-// half-warp one (fft_hw.cuh) for n_phi = 256, 384, 512, 768 and the block-wide
-// one (phi_fft.cuh) otherwise.
+// half-warp one (fft_hw.cuh) for n_phi = 256, 384, 512, 768, Stockham passes
+// (fft.cuh) for 250 and 500, and the two-step one (phi_fft.cuh) otherwise.
 #include "fft_hw.cuh"
 #include "phi_fft.cuh"
 #include "split_kernels.cuh"
@@ -216,6 +216,103 @@ __global__ void __launch_bounds__(kPhiThreads, SH::kMax <= 12 ? 4 : 3)
   }
 }
 
+// Rows of 125 = 25 x 5 points (n_phi 250 and 500): block-wide Stockham passes of
+// radices up to 8 (fft.cuh, kStRows rows at a time through a scratch buffer).  A row
+// has no more than ten 25-point transforms, each a long chain for one thread, and
+// three passes of radix 5 are as short as two steps.  A round of the four transforms
+// at n_phi 250, l_max 327, 7 columns: 333 us in two steps, 301 in passes; at n_phi
+// 500, l_max 163, 14 columns: 285 and 276; but at n_phi 800, l_max 266, 30 columns (20
+// x 10) 740 and 819, at n_phi 1000 (25 x 10), l_max 333, 1190 and 1328.
+constexpr int kStRows = 7;
+
+__global__ void __launch_bounds__(kPhiThreads) k_split_to_grid_st(SplitPhiArgs a) {
+  extern __shared__ __align__(16) float smemf[];
+  cplx<float>* buf = reinterpret_cast<cplx<float>*>(smemf);
+  const Tables& t = a.t;
+  const int N = t.n_phi, H = N / 2, M = t.n_m, nt = t.n_theta, S = padded_len(H);
+  const int row = blockIdx.x, j = row >> 1, tid = threadIdx.x;
+  const float hs = (row & 1) ? -1.f : 1.f;  // north = sym + asym, south = sym - asym
+  const int r0 = blockIdx.y * kPhiRows, nrow = min(kPhiRows, a.nrows - r0);
+  cplx<float>* tws = buf + (kPhiRows + kStRows) * S;
+  fft_twiddles_to_smem(tws, H, t.twiddle, t.fft_radix, t.fft_nstages);
+  const float* fs = a.Fs + (int64_t)j * a.fs_j + 2 * r0;
+  const float rcp = 1.0f / (float)nrow;
+  for (int e = tid; e < nrow * M; e += kPhiThreads) {
+    const int k = fdiv(e, rcp), q = e - k * nrow;
+    const float2 sy = __ldg(reinterpret_cast<const float2*>(fs + k * a.fs_m) + q);
+    const float2 as = __ldg(reinterpret_cast<const float2*>(fs + k * a.fs_m + a.fs_c) + q);
+    buf[q * S + pad16(k)] = {sy.x + hs * as.x, sy.y + hs * as.y};
+  }
+  for (int e = tid; e < nrow * (H - M); e += kPhiThreads) {
+    const int q = e / (H - M), k = M + e % (H - M);
+    buf[q * S + pad16(k)] = {0.f, 0.f};
+  }
+  __syncthreads();
+  // half spectrum -> Z in place (fft.cuh, c2r_pre), then the block FFT
+  for (int e = tid; e < nrow * (H / 2 + 1); e += kPhiThreads) {
+    const int q = e / (H / 2 + 1), k = e % (H / 2 + 1);
+    cplx<float>* rw = buf + q * S;
+    const int kc = H - k;
+    cplx<float> Xk = rw[pad16(k)];
+    if (k == 0) {
+      Xk.y = 0.f;
+      rw[pad16(0)] = c2r_pre(Xk, cplx<float>{0.f, 0.f}, 0, t.twiddle);
+    } else {
+      const cplx<float> Xc = rw[pad16(kc)];
+      const cplx<float> Zk = c2r_pre(Xk, Xc, k, t.twiddle);
+      const cplx<float> Zc = c2r_pre(Xc, Xk, kc, t.twiddle);
+      rw[pad16(k)] = Zk;
+      if (kc != k) rw[pad16(kc)] = Zc;
+    }
+  }
+  __syncthreads();
+  fft_rows<true>(buf, buf + kPhiRows * S, nrow, kStRows, H, S, t.fft_radix, t.fft_nstages, tws);
+  __syncthreads();
+  const int lane = tid & 31;
+  for (int q = tid >> 5; q < nrow; q += kPhiThreads / 32) {
+    const int r = r0 + q, b = r / a.nf, f = r - b * a.nf;
+    double2* dst = reinterpret_cast<double2*>(a.out[f] + ((int64_t)b * nt + row) * N);
+    for (int n = lane; n < H; n += 32) {
+      const cplx<float> z = buf[q * S + pad16(n)];
+      dst[n] = make_double2((double)z.x, (double)z.y);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kPhiThreads) k_split_to_fourier_st(SplitPhiArgs a) {
+  extern __shared__ __align__(16) float smemf[];
+  cplx<float>* buf = reinterpret_cast<cplx<float>*>(smemf);
+  const Tables& t = a.t;
+  const int N = t.n_phi, H = N / 2, M = t.n_m, nt = t.n_theta, S = padded_len(H);
+  const int row = blockIdx.x, j = row >> 1, tid = threadIdx.x, lane = tid & 31;
+  const int r0 = blockIdx.y * kPhiRows, nrow = min(kPhiRows, a.nrows - r0);
+  cplx<float>* tws = buf + (kPhiRows + kStRows) * S;
+  fft_twiddles_to_smem(tws, H, t.twiddle, t.fft_radix, t.fft_nstages);
+  for (int q = tid >> 5; q < nrow; q += kPhiThreads / 32) {
+    const int r = r0 + q, b = r / a.nf, f = r - b * a.nf;
+    const double2* src = reinterpret_cast<const double2*>(a.in[f] + ((int64_t)b * nt + row) * N);
+    for (int n = lane; n < H; n += 32) {
+      const double2 v = __ldg(src + n);
+      buf[q * S + pad16(n)] = {(float)v.x, (float)v.y};
+    }
+  }
+  __syncthreads();
+  fft_rows<false>(buf, buf + kPhiRows * S, nrow, kStRows, H, S, t.fft_radix, t.fft_nstages, tws);
+  __syncthreads();
+  const float ws = (float)(t.wq[row] / N), wv = (float)(t.wq_v[row] / N);
+  float* G = a.G + (int64_t)(row & 1) * a.g_h + (int64_t)j * a.g_j;
+  const float rcp = 1.0f / (float)nrow;
+  for (int e = tid; e < M * nrow; e += kPhiThreads) {
+    const int k = fdiv(e, rcp), q = e - k * nrow;
+    const int r = r0 + q, b = r / a.nf, f = r - b * a.nf;
+    const cplx<float>* z = buf + q * S;
+    const cplx<float> X = r2c_post(z[pad16(k)], z[pad16((H - k) % H)], k, t.twiddle);
+    const float w = (a.vector_mask >> f) & 1 ? wv : ws;
+    reinterpret_cast<float2*>(G + k * a.g_m + (int64_t)b * a.g_level)[f] =
+        make_float2(w * X.x, w * X.y);
+  }
+}
+
 template <typename K>
 static int launch_phi(K kern, size_t n_cplx, const SplitPhiArgs& a, cudaStream_t st) {
   const size_t sm = n_cplx * sizeof(cplx<float>);
@@ -240,6 +337,12 @@ static int launch_rows(bool to_grid, const SplitPhiArgs& a, cudaStream_t st) {
                  : launch_phi(k_split_to_fourier<SH>, n, a, st);
 }
 
+static int launch_st(bool to_grid, const SplitPhiArgs& a, cudaStream_t st) {
+  const int H = a.t.n_phi / 2;
+  const size_t n = (size_t)(kPhiRows + kStRows) * padded_len(H) + H;
+  return launch_phi(to_grid ? k_split_to_grid_st : k_split_to_fourier_st, n, a, st);
+}
+
 int launch_split_phi(bool to_grid, const SplitPhiArgs& a, cudaStream_t st) {
   switch (a.t.n_phi) {
     case 256: return launch_hw<8>(to_grid, a, st);
@@ -248,6 +351,7 @@ int launch_split_phi(bool to_grid, const SplitPhiArgs& a, cudaStream_t st) {
     case 768: return launch_hw<24>(to_grid, a, st);
     default: break;
   }
+  if (a.t.fft_a > 18 && a.t.fft_b <= 5) return launch_st(to_grid, a, st);
   return phi_max_radix(a.t) <= 12 ? launch_rows<PhiShapeRt<12>>(to_grid, a, st)
                                   : launch_rows<PhiShapeRt<27>>(to_grid, a, st);
 }
