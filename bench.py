@@ -191,14 +191,14 @@ class ClockSampler:
 
 
 # DRAM bytes (read + write) of one launch of the phi-stage kernel from an ncu
-# full-set capture of the same kernel at l_max = 255, n_r = 17, per Fourier row moved (13 fields x n_r in, 9 fields x (n_r - 2) out); traffic grows
+# capture of the same kernel at l_max = 255, n_r = 17, per Fourier row moved (13 fields x n_r in, 9 fields x (n_r - 2) out); traffic grows
 # in proportion to the rows, so the full-size launch is scaled by its row count.
-NCU_PHI_TRAFFIC = {"split": (230.161408e6 + 104.267520e6) / (13 * 17 + 9 * 15),
+NCU_PHI_TRAFFIC = {"split": (251.572224e6 + 101.860096e6) / (13 * 17 + 9 * 15),
                    # the FP64 phi kernel of the digit-split stage (k_nl_bouss)
-                   "ozaki": (347.744000e6 + 178.849280e6) / (13 * 17 + 9 * 15)}
+                   "ozaki": (348.220416e6 + 174.823680e6) / (13 * 17 + 9 * 15)}
 # warp instructions of the same launch (smsp__inst_executed.sum), per Fourier row
-NCU_PHI_INST = {"split": 184287744.0 / (13 * 17 + 9 * 15),
-                "ozaki": 209674368.0 / (13 * 17 + 9 * 15)}
+NCU_PHI_INST = {"split": 187290952.0 / (13 * 17 + 9 * 15),
+                "ozaki": 210501184.0 / (13 * 17 + 9 * 15)}
 
 
 def measured_peaks():
@@ -302,7 +302,8 @@ def run_anel(args, rank, world):
     perturbations |c_lm| ~ 1e-3 (l+1)^-2), through magic_b200.step.AnelasticStep
     with the stage of --precision (default the fused digit-split stage), beside
     the other two (unless --no-alt): the fused split-precision stage and the
-    FP64 stage (DMMA contractions and the FP64 phi kernel), all with the same FP64 solves; device-timed with the state resident (2.9 GB of spectral
+    FP64 stage (DMMA contractions and the FP64 phi kernel), all with the same
+    FP64 solves; device-timed with the state resident (2.9 GB of spectral
     arrays, larger than L2)."""
     from magic_b200.step import AnelasticStep
 

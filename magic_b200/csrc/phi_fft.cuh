@@ -17,9 +17,9 @@
 // kernels (its pipe was 60 % busy at n_phi = 768).  Measured against the passes
 // replaced: the FP64 Boussinesq phi stage at l_max 255 on 97 levels (n_phi 768,
 // warp FFTs) 2.74 -> 2.33 ms, the anelastic one at l_max 383 on 129 levels
-// (n_phi 1152, radix-8/3 stages) 9.16 -> 6.0 ms, the FP64 transforms of 37 columns
-// at l_max 213 (n_phi 640, out-of-place Stockham passes) 1.00 -> 0.73 ms in all;
-// 0.70 of the load/store pipe busy.
+// (n_phi 1152, radix-8/3 stages) 9.16 -> 5.8 ms, the FP64 transforms of 37 columns
+// at l_max 213 (n_phi 640, out-of-place Stockham passes) 1.00 -> 0.73 ms in all.
+// Shared memory is 55 % busy now, the FP64 pipe 36 %, at 16 warps an SM.
 //
 // Layout of a row: element (p, f, q) of wavenumber k = p F B + F q + f (outer
 // and inner step inputs) or of point (p, s = q, g = f) sits at
