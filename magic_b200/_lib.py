@@ -236,6 +236,36 @@ def check(rc):
         raise MagicError(f"magic_b200 status {rc}: {msg}")
 
 
+# torch carries out a conjugation or a sign lazily: x.conj() is a view of x's memory
+# with a bit set, and .to() and .contiguous() may hand the same memory back.  Kernels
+# read and write the memory.
+
+def plain(x):
+    """x as a kernel may read it: its memory holds its values."""
+    if x.is_conj():
+        x = x.resolve_conj()
+    return x.resolve_neg() if x.is_neg() else x
+
+
+def _flip(arrays):
+    for x in arrays:
+        if x.is_conj():
+            x.conj_physical_()
+        if x.is_neg():
+            x.neg_()
+
+
+def check_writes(arrays, call, *args):
+    """check(call(*args)) for a call that reads and writes the arrays in place: during
+    it, the memory of those with a lazy bit holds their values."""
+    lazy = [x for x in arrays if x.is_conj() or x.is_neg()]
+    _flip(lazy)
+    try:
+        check(call(*args))
+    finally:
+        _flip(lazy)
+
+
 # Codes the split-precision kernels record in the first int of their workspace
 # when a bounded wait runs out (the wait that gave up; see umma.cuh callers).
 DEVICE_STATUS = {

@@ -16,7 +16,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._lib import check
+from ._lib import check, check_writes, plain
 
 
 def cnab2_weights(dt1, dt2, alpha=0.6):
@@ -403,23 +403,24 @@ def update_poloidal_dc(plan, sch, lop, P0, w, dw, ddw, p, ta, weights, s, prof, 
     visc, dLvisc, ddLvisc, orho1, rgrav, rho0 over n_r (numpy or device arrays);
     P0: RadialOp of p0_inverse; wcoef: precomputed _w_coefficient_profiles(prof)."""
     n_r = w.shape[1]
-    arrs = [w, dw, ddw, ta["old"], ta["impl"], ta["expl0"], ta["expl1"], p, s]
-    for a in arrs + ([xi] if xi is not None else []):
+    arrs = [w, dw, ddw, ta["old"], ta["impl"], ta["expl0"], ta["expl1"], p]
+    for a in arrs + [s] + ([xi] if xi is not None else []):
         if a.shape != w.shape or a.dtype != torch.complex128 or not a.is_contiguous():
             raise ValueError("fields and time arrays must be contiguous (lm_max, n_r) complex128")
+    s, xi = plain(s), plain(xi) if xi is not None else None
     w_old, wimp_lin0, w_impl, w_e0, w_e1 = weights
     c3, c2n, c1n, c1d, c0n = wcoef if wcoef is not None else _w_coefficient_profiles(prof)
     prof_arrays = [hdif] + [prof[k] for k in (
         "or2", "orho1", "beta", "visc", "rgrav", "rho0")] + [c3, c2n, c1n, c1d, c0n]
     dev = [torch.as_tensor(v, dtype=torch.float64, device=w.device).contiguous()
            for v in prof_arrays]
-    u = _lib.PoloidalUpdate(*[a.data_ptr() for a in arrs],
+    u = _lib.PoloidalUpdate(*[a.data_ptr() for a in arrs], s.data_ptr(),
                             xi.data_ptr() if xi is not None else None, n_r,
                             w_old, w_impl, w_e0, w_e1, wimp_lin0, float(BuoFac), float(ChemFac),
                             *[d.data_ptr() for d in dev])
     st = C.c_void_p(torch.cuda.current_stream(w.device).cuda_stream)
-    check(_lib.lib().mt_update_poloidal(plan._h, n_r, C.byref(u), lop._h, sch.D1._h, sch.D2._h,
-                                        P0._h, st))
+    check_writes(arrs, _lib.lib().mt_update_poloidal, plan._h, n_r, C.byref(u), lop._h,
+                 sch.D1._h, sch.D2._h, P0._h, st)
 
 
 def update_wp(plan, sch, lop, P0, w, dw, ddw, p, dp, taw, tap, weights, s, prof, hdif,
@@ -436,21 +437,23 @@ def update_wp(plan, sch, lop, P0, w, dw, ddw, p, dp, taw, tap, weights, s, prof,
     constraint; None: p = 0 at the outer boundary."""
     n_r = w.shape[1]
     arrs = [w, dw, ddw, p, dp, taw["old"], taw["impl"], taw["expl0"], taw["expl1"], tap["old"],
-            tap["impl"], tap["expl0"], tap["expl1"], s]
-    for a in arrs + ([xi] if xi is not None else []):
+            tap["impl"], tap["expl0"], tap["expl1"]]
+    for a in arrs + [s] + ([xi] if xi is not None else []):
         if a.shape != w.shape or a.dtype != torch.complex128 or not a.is_contiguous():
             raise ValueError("fields and time arrays must be contiguous (lm_max, n_r) complex128")
+    s, xi = plain(s), plain(xi) if xi is not None else None
     w_old, wimp_lin0, w_impl, w_e0, w_e1 = weights
     dev = [torch.as_tensor(v, dtype=torch.float64, device=w.device).contiguous()
            for v in [hdif] + [prof[k] for k in ("or1", "or2", "beta", "dbeta", "visc", "dLvisc",
                                                "rgrav", "rho0")]]
-    u = _lib.WpUpdate(*[a.data_ptr() for a in arrs], xi.data_ptr() if xi is not None else None,
-                      n_r, w_old, w_impl, w_e0, w_e1, wimp_lin0, float(BuoFac), float(ChemFac),
+    u = _lib.WpUpdate(*[a.data_ptr() for a in arrs], s.data_ptr(),
+                      xi.data_ptr() if xi is not None else None, n_r, w_old, w_impl, w_e0,
+                      w_e1, wimp_lin0, float(BuoFac), float(ChemFac),
                       *[d.data_ptr() for d in dev], int(bool(impl_interior)),
                       p0_row0.data_ptr() if p0_row0 is not None else None)
     st = C.c_void_p(torch.cuda.current_stream(w.device).cuda_stream)
-    check(_lib.lib().mt_update_wp(plan._h, n_r, C.byref(u), lop._h, sch.D1._h, sch.D2._h,
-                                  sch.D3._h, P0._h, st))
+    check_writes(arrs, _lib.lib().mt_update_wp, plan._h, n_r, C.byref(u), lop._h, sch.D1._h,
+                 sch.D2._h, sch.D3._h, P0._h, st)
 
 
 def entropy_coefficients(l_max, opr, hdif, kappa, d1c, or2):
@@ -535,6 +538,7 @@ def update_field(plan, sch, lop, x, dx, ta, weights, coef, top=None, bot=None, d
     if d2x is not None and (d2x.shape != x.shape or d2x.dtype != torch.complex128
                             or not d2x.is_contiguous()):
         raise ValueError("d2x must be a contiguous (lm_max, n_r) complex128 array")
+    top, bot = (plain(v) if v is not None else None for v in (top, bot))
     u = _lib.FieldUpdate(arrs[0].data_ptr(), arrs[1].data_ptr(),
                          d2x.data_ptr() if d2x is not None else None,
                          *[a.data_ptr() for a in arrs[2:]],
@@ -543,7 +547,8 @@ def update_field(plan, sch, lop, x, dx, ta, weights, coef, top=None, bot=None, d
                          w_old, w_impl, w_e0, w_e1,
                          *[dev[k].data_ptr() if dev[k] is not None else None for k in names])
     st = C.c_void_p(torch.cuda.current_stream(x.device).cuda_stream)
-    check(_lib.lib().mt_update_field(plan._h, n_r, C.byref(u), lop._h, sch.D1._h, sch.D2._h, st))
+    check_writes(arrs + ([d2x] if d2x is not None else []), _lib.lib().mt_update_field, plan._h,
+                 n_r, C.byref(u), lop._h, sch.D1._h, sch.D2._h, st)
 
 
 def am_profiles(r, rho0, beta, dbeta, rint):
@@ -568,7 +573,8 @@ def correct_am(plan, z, dz, ta, coef, am, d2z=None):
     n_r = z.shape[1]
     names = ("so_l", "so_r", "ia_l", "ia_r", "ib_r", "ic_r", "ic_l", "ic_r2")
     ptr = lambda x: x.data_ptr() if x is not None else None
-    for a in (z, dz, ta["old"], ta["impl"]):
+    arrs = [z, dz, ta["old"], ta["impl"]]
+    for a in arrs:
         if a.shape != z.shape or a.dtype != torch.complex128 or not a.is_contiguous():
             raise ValueError("fields and time arrays must be contiguous (lm_max, n_r) complex128")
     u = _lib.FieldUpdate(z.data_ptr(), dz.data_ptr(), ptr(d2z), ta["old"].data_ptr(),
@@ -578,7 +584,8 @@ def correct_am(plan, z, dz, ta, coef, am, d2z=None):
                           float(am["c_moi_oc"]), float(am["am_start"]), int(am["axial"]),
                           int(am["equatorial"]))
     st = C.c_void_p(torch.cuda.current_stream(z.device).cuda_stream)
-    check(_lib.lib().mt_correct_am(plan._h, n_r, C.byref(u), C.byref(c), st))
+    check_writes(arrs + ([d2z] if d2z is not None else []), _lib.lib().mt_correct_am, plan._h,
+                 n_r, C.byref(u), C.byref(c), st)
 
 
 def update_scalar(plan, sch, lop, s, ds, ta, weights, opr, hdif, kappa, d1c, or2, top=None,

@@ -16,7 +16,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._lib import check
+from ._lib import check, plain
 
 EKin = namedtuple("EKin", "e_p e_t e_p_as e_t_as e_p_es e_t_es e_p_eas e_t_eas")
 EMagOC = namedtuple("EMagOC", "e_p e_t e_p_as e_t_as e_p_os e_p_as_os "
@@ -49,6 +49,9 @@ class EnergyIntegrals:
                 raise ValueError("fields must be (lm_max, n_r) complex128 with unit radial stride")
         if not (pol.stride(0) == dpol.stride(0) == tor.stride(0)):
             raise ValueError("fields must share their row stride")
+        pol, dpol, tor = plain(pol), plain(dpol), plain(tor)
+        if not (pol.stride(0) == dpol.stride(0) == tor.stride(0)):
+            pol, dpol, tor = pol.contiguous(), dpol.contiguous(), tor.contiguous()
         out = torch.empty(10, dtype=torch.float64, device=self.plan.device)
         e = _lib.EnergyArgs(pol.data_ptr(), dpol.data_ptr(), tor.data_ptr(), pol.stride(0),
                             self.or2.data_ptr(), cr.data_ptr(), self.rint.data_ptr(),

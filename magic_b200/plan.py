@@ -16,7 +16,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._lib import MagicError, check, raise_device_status
+from ._lib import MagicError, check, check_writes, plain, raise_device_status
 
 _CD = torch.complex128
 _RD = torch.float64
@@ -178,6 +178,7 @@ class Plan:
             raise ValueError(f"{name}: expected shape (lm_max={self.lm_max},[B])")
         if x.dtype != _CD:
             x = x.to(_CD)
+        x = plain(x)
         if n == 1:
             if x.stride(0) < 1:
                 x = x.contiguous()
@@ -195,7 +196,7 @@ class Plan:
             raise ValueError(f"{name}: expected shape ([B,] {self.n_theta_max}, {self.n_phi_max})")
         if x.dtype != _RD:
             x = x.to(_RD)
-        return x.contiguous(), x.size(0) if n == 3 else 1, n == 2
+        return plain(x).contiguous(), x.size(0) if n == 3 else 1, n == 2
 
     def _new_grid(self, B, one):
         shape = (self.n_theta_max, self.n_phi_max)
@@ -292,14 +293,14 @@ class Plan:
             if a.shape != (n_r, self.n_theta_max, self.n_phi_max) or a.device != self.device:
                 raise ValueError(f"{name}[{i}]: expected ({n_r}, {self.n_theta_max}, "
                                  f"{self.n_phi_max}) on {self.device}")
-            out.append(a.to(_RD).contiguous())
+            out.append(plain(a.to(_RD)).contiguous())
         return out
 
     def _prof(self, x, n_r):
         t = torch.as_tensor(x, dtype=_RD, device=self.device).reshape(-1)
         if t.numel() == 1 and n_r > 1:
             t = t.expand(n_r)
-        return t.contiguous()
+        return plain(t).contiguous()
 
     def get_nl(self, grids, or2, or4, LFfac):
         """get_nl products (magic_torch/get_nl.py:30-87); grids: 14 (n_r, nt, np)."""
@@ -374,7 +375,7 @@ class Plan:
             x = fields[k]
             if x.shape != (self.lm_max, n_r) or x.dtype != _CD or x.device != self.device:
                 raise ValueError(f"fields[{k}]: expected ({self.lm_max}, {n_r}) complex128")
-            ins[k] = x.contiguous()
+            ins[k] = plain(x).contiguous()
         onames = ["Advr", "Advt", "Advp", "VSr", "VSt"] + (["VxBr", "VxBt", "VxBp"] if l_mag
                                                            else []) + \
             (["VXir", "VXit"] if l_chem else [])
@@ -403,8 +404,9 @@ class Plan:
         need = L.mt_nl_bouss_workspace(self._h, n_r, int(l_mag), int(l_chem))
         if work is None or work.numel() < need:
             work = self._work(need)
-        check(L.mt_nl_bouss(self._h, n_r, C.byref(bi), C.byref(bo), C.byref(bp), _ptr(dtr),
-                            _ptr(dth), _ptr(work), work.numel(), self._stream()))
+        check_writes([out[k] for k in onames if k in out], L.mt_nl_bouss, self._h, n_r,
+                     C.byref(bi), C.byref(bo), C.byref(bp), _ptr(dtr), _ptr(dth), _ptr(work),
+                     work.numel(), self._stream())
         self._watch(work, "nl_bouss", fused=True)
         return out, dtr, dth
 
@@ -434,7 +436,7 @@ class Plan:
             x = ins[k]
             if x.shape != (self.lm_max, n_r) or x.dtype != _CD or x.device != self.device:
                 raise ValueError(f"ins[{k}]: expected ({self.lm_max}, {n_r}) complex128")
-            src[k] = x.contiguous()
+            src[k] = plain(x).contiguous()
         onames = ["dwdt", "dzdt"] + ([] if l_double_curl else ["dpdt"]) + \
             (["dsdt"] if l_heat else []) + (["dxidt"] if l_chem else []) + \
             (["dbdt", "djdt"] if l_mag else [])
@@ -453,8 +455,9 @@ class Plan:
                                                           "beta")],
                            float(CorFac), int(l_double_curl), int(l_heat), int(l_mag),
                            int(l_chem), int(l_anel))
-        check(_lib.lib().mt_get_td(self._h, n_r, C.byref(ti), C.byref(to), C.byref(tp),
-                                   D1._h if D1 is not None else None, self._stream()))
+        check_writes([out[k] for k in onames if k in out], _lib.lib().mt_get_td, self._h, n_r,
+                     C.byref(ti), C.byref(to), C.byref(tp), D1._h if D1 is not None else None,
+                     self._stream())
         return out
 
     def nl_anel_workspace(self, n_r, l_mag=True, l_chem=False):
@@ -486,7 +489,7 @@ class Plan:
             x = fields[k]
             if x.shape != (self.lm_max, n_r) or x.dtype != _CD or x.device != self.device:
                 raise ValueError(f"fields[{k}]: expected ({self.lm_max}, {n_r}) complex128")
-            ins[k] = x.resolve_conj().contiguous()
+            ins[k] = plain(x).contiguous()
         need = self.nl_anel_workspace(n_r, l_mag, l_chem) if n_r >= 3 else 0
         if need == 0:
             raise MagicError("nl_anel needs n_r >= 3")
@@ -502,7 +505,7 @@ class Plan:
             o0 = out[onames[0]]
             fits = all(x.shape == (self.lm_max, n_r) and x.dtype == _CD
                        and x.device == self.device and x.stride(1) == 1
-                       and x.stride(0) == o0.stride(0) >= n_r and not x.is_conj()
+                       and x.stride(0) == o0.stride(0) >= n_r
                        for x in (out[k] for k in onames))
             if not fits:
                 out = {k: torch.empty(self.lm_max, n_r, dtype=_CD, device=self.device)
@@ -528,8 +531,9 @@ class Plan:
         if work is None or work.numel() < need:
             work = self._work(need)
         run = L.mt_nl_anel_f64 if self.precision == "fp64" else L.mt_nl_anel
-        check(run(self._h, n_r, C.byref(ai), C.byref(ao), C.byref(ap), _ptr(dtr), _ptr(dth),
-                  _ptr(work), work.numel(), self._stream()))
+        check_writes([out[k] for k in onames if k in out], run, self._h, n_r, C.byref(ai),
+                     C.byref(ao), C.byref(ap), _ptr(dtr), _ptr(dth), _ptr(work), work.numel(),
+                     self._stream())
         self._watch(work, "nl_anel", fused=True)
         if out is not given:
             for k in onames:

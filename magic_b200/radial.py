@@ -21,7 +21,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._lib import check
+from ._lib import check, plain
 
 _CD = torch.complex128
 
@@ -243,7 +243,7 @@ class RadialOp:
     def _rows(self, f):
         if f.dtype != _CD or f.device != self.device or f.shape[-1] != self.n_r:
             raise ValueError(f"expected complex128 (..., {self.n_r}) on {self.device}")
-        return f.contiguous()
+        return plain(f).contiguous()
 
     def __call__(self, f):
         f = self._rows(f)
