@@ -1217,18 +1217,23 @@ __global__ void __launch_bounds__(kWpThreads) k_update_wp(WpArgs a) {
   }
 }
 
-// The same update with the coupled solve on the FP64 tensor pipe, for 144 < n_r
-// <= 192 (or operators that are not dense): CTA = 16 orders (4 m-tiles) of one
-// degree, 9 warps, at most kNt = 6 n-tiles of 8 levels per warp.  The rows'
-// right-hand sides (w part, then p part, row stride fs) are the A operand of
-// solve_tile_dmma with the 2 n_r x 2 n_r operator streamed through shared
-// memory in 16-row chunks; the solution overwrites them.  Derivatives: thread =
-// (4-row group, level), each D coefficient serving 4 rows.
+// The same update with the coupled solve on the FP64 tensor pipe and the
+// derivatives by op_rows_wp, for derivative operators that are banded and for the
+// sizes where it is the faster one (mt_update_wp).  CTA = 16 orders (4 m-tiles) of
+// one degree; the rows' right-hand sides (w part, then p part, row stride fs) are
+// the A operand of solve_tile_dmma with the 2 n_r x 2 n_r operator streamed through
+// shared memory in 16-row chunks; the solution overwrites them.  Derivatives:
+// thread = (4-row group, level), each D coefficient serving 4 rows.  Up to 128
+// levels 8 warps with at most kNt = 4 n-tiles of 8 levels each, two CTAs an SM;
+// above, up to 192, 9 warps with six, one CTA (its shared memory allows no more).
+// With banded operators the second CTA takes the update at l_max 213 on 73 levels
+// from 341 to 222 us, on 128 levels from 606 to 575.
+constexpr int kWpDmmaMaxR = 128;
 constexpr int kWpDmmaWideMaxR = 192;
-constexpr int kWpDmmaThreads = 288;
+__host__ __device__ constexpr int wp_dmma_threads(int kNt) { return kNt == 4 ? 256 : 288; }
 
 template <int kNt>
-__global__ void __launch_bounds__(kWpDmmaThreads, 1)
+__global__ void __launch_bounds__(wp_dmma_threads(kNt), kNt == 4 ? 2 : 1)
     k_update_wp_dmma(WpArgs a, int fs) {
   extern __shared__ __align__(16) double2 wpd[];
   __shared__ int lm_row[4 * kRows];
@@ -1939,10 +1944,11 @@ int mt_update_wp(const mt_plan* p, int n_r, const mt_wp_update* u, const mt_lop*
     const int fs = 2 * n_r + ((4 - 2 * n_r) & 7);
     const size_t sm = (size_t)4 * kRows * fs * sizeof(double2) +
                       (size_t)2 * kKc * a.ldm * sizeof(double);
-    auto kern = k_update_wp_dmma<6>;
+    const bool narrow = n_r <= kWpDmmaMaxR;
+    auto kern = narrow ? k_update_wp_dmma<4> : k_update_wp_dmma<6>;
     MT_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     const dim3 grid((p->n_m + 4 * kRows - 1) / (4 * kRows), p->l_max + 1);
-    kern<<<grid, kWpDmmaThreads, sm, (cudaStream_t)stream>>>(a, fs);
+    kern<<<grid, wp_dmma_threads(narrow ? 4 : 6), sm, (cudaStream_t)stream>>>(a, fs);
     MT_CHECK_CUDA(cudaGetLastError());
     return MT_OK;
   }

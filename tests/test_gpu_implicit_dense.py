@@ -131,3 +131,30 @@ def test_wp_update(n_r, interior):
     got.update({f"w_{k}": gw[k] for k in ("old", "impl", "expl1")},
                **{f"p_{k}": gp[k] for k in ("old", "impl", "expl1")})
     _check(got, ref)
+
+
+def _banded(rng, n):
+    """A random operator with a band of two on either side (one-sided at the ends)."""
+    D = np.zeros((n, n))
+    for j in range(n):
+        k = min(max(j - 2, 0), max(n - 5, 0))
+        D[j, k:k + 5] = rng.standard_normal(min(5, n))
+    return D
+
+
+@pytest.mark.parametrize("n_r", [7, 16, 65, 128, 129, 192, 193])
+def test_wp_update_banded_derivatives(n_r, monkeypatch):
+    """Banded derivative operators take the other form of the coupled solve, with two
+    limits (128 and 192 levels)."""
+    dense = _setup
+
+    def banded(l_max, minc, n, seed):
+        from magic_b200.radial import RadialOp
+
+        rng, plan, _, _, cplx, vec = dense(l_max, minc, n, seed)
+        D = [_banded(rng, n) for _ in range(3)]
+        sch = types.SimpleNamespace(**{f"D{i + 1}": RadialOp(D[i]) for i in range(3)})
+        return rng, plan, [torch.from_numpy(d) for d in D], sch, cplx, vec
+
+    monkeypatch.setitem(globals(), "_setup", banded)
+    test_wp_update(n_r, False)
