@@ -38,6 +38,9 @@ void set_error(const std::string& msg);
 
 constexpr int kMaxFftStages = 24;
 
+// SMs of a B200, as a measure of waves (persistent grids ask the device).
+constexpr int kSms = 148;
+
 // Device-side view of the horizontal tables, passed by value to kernels.
 struct Tables {
   int l_max, minc, n_theta, n_phi, n_m, lm_max, nhs;

@@ -765,6 +765,13 @@ __device__ __forceinline__ void dn_zero(double (&acc)[kNt][4][2]) {
     for (int t = 0; t < 4; ++t) acc[i][t][0] = acc[i][t][1] = 0.0;
 }
 
+// CTAs of 16 orders with work: the orders m <= l of every degree.
+int dn_ctas(int l_max, int minc) {
+  int n = 0;
+  for (int l = 0; l <= l_max; ++l) n += (l / minc + 4 * kRows) / (4 * kRows);
+  return n;
+}
+
 // accumulators of the solve over the right-hand sides in f (imaginary part of
 // m = 0 dropped)
 template <int kNt>
@@ -1291,6 +1298,22 @@ __global__ void __launch_bounds__(wp_dmma_threads(kNt), kNt == 4 ? 2 : 1)
                d1[r], d2[r], d3[r], dp[r]);
     }
   }
+}
+
+// Which coupled updates with dense operators run as one chain (below), of nt_s
+// n-tiles (2 n_r / 8) up to 36, chain and other form (k_update_wp_dmma, two CTAs an
+// SM) at each line:
+//   10 to 12 tiles: three CTAs of five or six warps an SM, which pay where they save
+//   a wave: at 48 levels 38 and 55 us (l_max 96), but 36 and 33 (64), 74 and 67 (127);
+//   19 to 27 tiles but 24: one CTA, its warps unevenly loaded, against two, the more
+//   so the more waves there are: at 73 levels 76 and 72 us (l_max 64), 462 and 394
+//   (213), at 97 levels 435 and 441 (170), 664 and 640 (213); but where the grid does
+//   not fill the SMs once, 42 and 54 (l_max 32, 73 levels).
+bool wp_chain(int nt_s, int ctas) {
+  const auto waves = [&](int per_sm) { return (ctas + per_sm * kSms - 1) / (per_sm * kSms); };
+  if (nt_s >= 10 && nt_s <= 12) return ctas <= kSms || waves(3) < waves(2);
+  if (nt_s >= 19 && nt_s <= 27 && nt_s != 24) return ctas <= (nt_s <= 23 ? kSms : 8 * kSms);
+  return nt_s <= 36;
 }
 
 // The same update with everything on the FP64 tensor pipe (dense D1, D2, D3; see
@@ -1926,7 +1949,7 @@ int mt_update_wp(const mt_plan* p, int n_r, const mt_wp_update* u, const mt_lop*
   a.D3 = radial_op_view(D3);
   a.P0 = radial_op_view(P0);
   const int nt_s = (2 * n_r + 7) / 8, tiles = (nt_s + kDnMaxTiles - 1) / kDnMaxTiles;
-  if (tiles <= 4 && D1->dense && D2->dense && D3->dense) {  // n_r <= 144
+  if (D1->dense && D2->dense && D3->dense && wp_chain(nt_s, dn_ctas(p->l_max, p->minc))) {
     const int fs = 2 * n_r + ((4 - 2 * n_r) & 7);
     a.ldd = lop_ld(n_r);
     const int ring = kKc * std::max(a.ldm, 2 * a.ldd);

@@ -401,11 +401,11 @@ def test_update_wp_matches_reference():
                                                          (16, 1, 129, 2, 1e2),
                                                          (8, 1, 193, 2, 3e3)])
 def test_update_wp_vs_oracle(l_max, minc, n_r, ktopv, scale):
-    """l_max = 127 on 65 Chebyshev levels (no-slip) and l_max = 32, minc = 4 on 33
-    levels (stress-free) with anelastic-like profiles, against the oracle's LU
-    solves (the tensor-pipe tiling with four n-tiles per warp, n_r <= 128);
-    l_max = 16 on 129 levels takes the six-tile variant (n_r <= 192, the
-    anelastic benchmark's levels), l_max = 8 on 193 levels the FMA tiling.  The
+    """l_max = 127 on 65 Chebyshev levels (no-slip), l_max = 32, minc = 4 on 33
+    levels (stress-free) and l_max = 16 on 129 levels (the anelastic benchmark's)
+    with anelastic-like profiles, against the oracle's LU solves: the chain of
+    contractions with two and four n-tiles per warp; l_max = 8 on 193 levels takes
+    the FMA tiling.  The
     coupled Chebyshev operator is far worse conditioned than the scalar ones (its
     p rows carry d3rMat): the tolerances are relative to each array's largest
     value, 1e-11 for the fields and 1e-10 for the terms that apply D2 / D3 to the
@@ -445,3 +445,10 @@ def test_update_wp_vs_oracle(l_max, minc, n_r, ktopv, scale):
     for k, v in errs.items():
         assert v < scale * (1e-10 if k in ("ddw", "w_impl", "p_impl", "p_old", "dw", "dp")
                             else 1e-11), (k, v)
+
+
+def test_update_wp_uneven_tiles_vs_oracle():
+    """81 levels at l_max = 64 (more CTAs than SMs): the solve with four n-tiles per
+    warp and dense derivatives by FMAs.  Scale 10: the conditioning's (81 / 65)^4 and
+    the D3 norm's (81 / 65)^6 are 2.4 and 3.7 times those at 65 levels."""
+    test_update_wp_vs_oracle(64, 1, 81, 2, 1e1)
