@@ -772,6 +772,16 @@ int dn_ctas(int l_max, int minc) {
   return n;
 }
 
+// Which field updates with dense operators run as one chain.  Up to 144 levels two
+// or three CTAs share an SM, above it one does.  There, up to 170 levels, the form
+// with the derivatives by FMAs holds three groups of rows a CTA and two CTAs an SM
+// and takes a grid of one to three waves of SMs in fewer of them: chain and other
+// form at 145 levels 91 and 81 us (l_max 64), 144 and 129 (96), but 200 and 228 (127),
+// 347 and 346 (170).
+bool field_chain(int n_r, int ctas) {
+  return n_r <= 144 || n_r > 170 || ctas <= kSms || ctas > 3 * kSms;
+}
+
 // accumulators of the solve over the right-hand sides in f (imaginary part of
 // m = 0 dropped)
 template <int kNt>
@@ -1772,7 +1782,8 @@ int mt_update_field(const mt_plan* p, int n_r, const mt_field_update* u, const m
   a.band = BandView{solve->abd, solve->piv, solve->fr, solve->fc, solve->kl, solve->ku, nullptr};
   a.D1 = radial_op_view(D1);
   a.D2 = radial_op_view(D2);
-  if (!solve->abd && n_r <= kStagedMaxR && D1->dense && D2->dense) {
+  if (!solve->abd && n_r <= kStagedMaxR && D1->dense && D2->dense &&
+      field_chain(n_r, dn_ctas(p->l_max, p->minc))) {
     const int nt_n = (n_r + 7) / 8, tiles = (nt_n + kDnMaxTiles - 1) / kDnMaxTiles;
     a.fs = n_r + ((4 - n_r) & 7);  // conflict-free A fragments
     const size_t sm = (size_t)4 * kRows * a.fs * sizeof(double2) +

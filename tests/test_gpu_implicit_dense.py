@@ -158,3 +158,10 @@ def test_wp_update_banded_derivatives(n_r, monkeypatch):
 
     monkeypatch.setitem(globals(), "_setup", banded)
     test_wp_update(n_r, False)
+
+
+@pytest.mark.parametrize("n_r", [144, 145, 170, 171])
+def test_field_update_on_few_waves(n_r):
+    """l_max 64 is 165 CTAs: between one and three waves of SMs the derivatives of 145
+    to 170 levels run by FMAs."""
+    test_field_update(n_r, 64, 1)
