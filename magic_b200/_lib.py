@@ -7,6 +7,8 @@ fallback: if the library is missing or cannot be loaded, ``lib()`` raises.
 import ctypes as C
 import os
 
+import torch
+
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libmagic_b200.so")
 
@@ -234,6 +236,18 @@ def check(rc):
     if rc != MT_OK:
         msg = lib().mt_last_error().decode(errors="replace")
         raise MagicError(f"magic_b200 status {rc}: {msg}")
+
+
+# torch's own call for a stream's handle, which builds no torch.cuda.Stream; it is not
+# a documented one, so the documented one stands in where a torch has none.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
+def stream_handle(device):
+    """Handle of the current stream of a CUDA device (with an index)."""
+    if _raw_stream is None:
+        return torch.cuda.current_stream(device).cuda_stream
+    return _raw_stream(device.index)
 
 
 # torch carries out a conjugation or a sign lazily: x.conj() is a view of x's memory

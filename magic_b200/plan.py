@@ -164,7 +164,7 @@ class Plan:
     # torch.cuda.Stream, addresses as plain integers, and results allocated in the
     # shape that is returned instead of a view of a larger one.
     def _stream(self):
-        return torch._C._cuda_getCurrentRawStream(self.device.index)
+        return _lib.stream_handle(self.device)
 
     def _work(self, nbytes):
         return torch.empty(max(int(nbytes), 16), dtype=torch.uint8, device=self.device)

@@ -45,3 +45,19 @@ def test_fused_stage_calls_mark_themselves_fused():
     for name in ("nl_bouss", "nl_anel"):
         src = inspect.getsource(getattr(Plan, name))
         assert f'self._watch(work, "{name}", fused=True)' in src, name
+
+
+def test_stream_handle_without_the_undocumented_call(monkeypatch):
+    """A torch without it: the documented call gives the handle."""
+    import types
+
+    import torch
+
+    from magic_b200 import _lib
+
+    p = _plan("fp64")
+    p.device = torch.device("cuda", 3)
+    monkeypatch.setattr(_lib, "_raw_stream", None)
+    monkeypatch.setattr(torch.cuda, "current_stream",
+                        lambda d: types.SimpleNamespace(cuda_stream=100 + d.index))
+    assert p._stream() == 103
