@@ -19,6 +19,14 @@ from . import _lib
 from ._lib import check, check_writes, plain
 
 
+def _coefs(v, device):
+    """A coefficient array as the kernels read it: float64, contiguous, on the device."""
+    if isinstance(v, torch.Tensor) and v.dtype == torch.float64 and v.device == device and \
+            v.is_contiguous() and not v.is_neg():
+        return v
+    return plain(torch.as_tensor(v, dtype=torch.float64, device=device)).contiguous()
+
+
 def cnab2_weights(dt1, dt2, alpha=0.6):
     """(w_old, w_impl_now, w_impl_prev, w_expl0, w_expl1) of CNAB2 with time steps
     dt1 (current) and dt2 (previous) (magic_torch/time_scheme.py:56-73):
@@ -412,13 +420,12 @@ def update_poloidal_dc(plan, sch, lop, P0, w, dw, ddw, p, ta, weights, s, prof, 
     c3, c2n, c1n, c1d, c0n = wcoef if wcoef is not None else _w_coefficient_profiles(prof)
     prof_arrays = [hdif] + [prof[k] for k in (
         "or2", "orho1", "beta", "visc", "rgrav", "rho0")] + [c3, c2n, c1n, c1d, c0n]
-    dev = [torch.as_tensor(v, dtype=torch.float64, device=w.device).contiguous()
-           for v in prof_arrays]
+    dev = [_coefs(v, w.device) for v in prof_arrays]
     u = _lib.PoloidalUpdate(*[a.data_ptr() for a in arrs], s.data_ptr(),
                             xi.data_ptr() if xi is not None else None, n_r,
                             w_old, w_impl, w_e0, w_e1, wimp_lin0, float(BuoFac), float(ChemFac),
                             *[d.data_ptr() for d in dev])
-    st = C.c_void_p(torch.cuda.current_stream(w.device).cuda_stream)
+    st = _lib.stream_handle(w.device)
     check_writes(arrs, _lib.lib().mt_update_poloidal, plan._h, n_r, C.byref(u), lop._h,
                  sch.D1._h, sch.D2._h, P0._h, st)
 
@@ -443,7 +450,7 @@ def update_wp(plan, sch, lop, P0, w, dw, ddw, p, dp, taw, tap, weights, s, prof,
             raise ValueError("fields and time arrays must be contiguous (lm_max, n_r) complex128")
     s, xi = plain(s), plain(xi) if xi is not None else None
     w_old, wimp_lin0, w_impl, w_e0, w_e1 = weights
-    dev = [torch.as_tensor(v, dtype=torch.float64, device=w.device).contiguous()
+    dev = [_coefs(v, w.device)
            for v in [hdif] + [prof[k] for k in ("or1", "or2", "beta", "dbeta", "visc", "dLvisc",
                                                "rgrav", "rho0")]]
     u = _lib.WpUpdate(*[a.data_ptr() for a in arrs], s.data_ptr(),
@@ -451,7 +458,7 @@ def update_wp(plan, sch, lop, P0, w, dw, ddw, p, dp, taw, tap, weights, s, prof,
                       w_e1, wimp_lin0, float(BuoFac), float(ChemFac),
                       *[d.data_ptr() for d in dev], int(bool(impl_interior)),
                       p0_row0.data_ptr() if p0_row0 is not None else None)
-    st = C.c_void_p(torch.cuda.current_stream(w.device).cuda_stream)
+    st = _lib.stream_handle(w.device)
     check_writes(arrs, _lib.lib().mt_update_wp, plan._h, n_r, C.byref(u), lop._h, sch.D1._h,
                  sch.D2._h, sch.D3._h, P0._h, st)
 
@@ -533,8 +540,7 @@ def update_field(plan, sch, lop, x, dx, ta, weights, coef, top=None, bot=None, d
             raise ValueError("fields and time arrays must be contiguous (lm_max, n_r) complex128")
     w_old, _, w_impl, w_e0, w_e1 = weights
     names = ("so_l", "so_r", "ia_l", "ia_r", "ib_r", "ic_r", "ic_l", "ic_r2")
-    dev = {k: (torch.as_tensor(coef[k], dtype=torch.float64, device=x.device).contiguous()
-               if coef.get(k) is not None else None) for k in names}
+    dev = {k: _coefs(coef[k], x.device) if coef.get(k) is not None else None for k in names}
     if d2x is not None and (d2x.shape != x.shape or d2x.dtype != torch.complex128
                             or not d2x.is_contiguous()):
         raise ValueError("d2x must be a contiguous (lm_max, n_r) complex128 array")
@@ -546,7 +552,7 @@ def update_field(plan, sch, lop, x, dx, ta, weights, coef, top=None, bot=None, d
                          bot.data_ptr() if bot is not None else None, n_r,
                          w_old, w_impl, w_e0, w_e1,
                          *[dev[k].data_ptr() if dev[k] is not None else None for k in names])
-    st = C.c_void_p(torch.cuda.current_stream(x.device).cuda_stream)
+    st = _lib.stream_handle(x.device)
     check_writes(arrs + ([d2x] if d2x is not None else []), _lib.lib().mt_update_field, plan._h,
                  n_r, C.byref(u), lop._h, sch.D1._h, sch.D2._h, st)
 
@@ -583,7 +589,7 @@ def correct_am(plan, z, dz, ta, coef, am, d2z=None):
     c = _lib.AmCorrection(*[am[k].data_ptr() for k in ("rint", "r", "am_z", "am_dz", "am_d2z")],
                           float(am["c_moi_oc"]), float(am["am_start"]), int(am["axial"]),
                           int(am["equatorial"]))
-    st = C.c_void_p(torch.cuda.current_stream(z.device).cuda_stream)
+    st = _lib.stream_handle(z.device)
     check_writes(arrs + ([d2z] if d2z is not None else []), _lib.lib().mt_correct_am, plan._h,
                  n_r, C.byref(u), C.byref(c), st)
 
