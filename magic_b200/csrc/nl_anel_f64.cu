@@ -126,8 +126,12 @@ static int launch_nl_anel_f64_s(const NlAnelArgs& a, cudaStream_t st) {
 
 template <bool MAG, bool CHEM>
 static int launch_nl_anel_f64_t(const NlAnelArgs& a, cudaStream_t st) {
-  if (phi_shape_is<16, 18, 2>(a.t))  // n_phi = 1152
-    return launch_nl_anel_f64_s<MAG, CHEM, PhiShape<16, 18, 2>>(a, st);
+  if (phi_shape_static(a.t)) switch (a.t.fft_b) {
+#define X(b) case b: return launch_nl_anel_f64_s<MAG, CHEM, PhiShape<16, b, 2>>(a, st);
+      MT_PHI_STATIC_B(X)
+#undef X
+      default: break;
+    }
   const int r = phi_max_radix(a.t);
   if (r <= 12) return launch_nl_anel_f64_s<MAG, CHEM, PhiShapeRt<12>>(a, st);
   return r <= 18 ? launch_nl_anel_f64_s<MAG, CHEM, PhiShapeRt<18>>(a, st)

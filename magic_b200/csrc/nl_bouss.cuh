@@ -133,10 +133,13 @@ static int launch_nl_bouss_s(const NlBoussArgs& a, cudaStream_t st) {
 
 template <bool MAG, bool CHEM, bool SPLIT_IO>
 static int launch_nl_bouss_t(const NlBoussArgs& a, cudaStream_t st) {
-  if (phi_shape_is<16, 12, 2>(a.t))  // n_phi = 768
-    return launch_nl_bouss_s<MAG, CHEM, SPLIT_IO, PhiShape<16, 12, 2>, 256>(a, st);
-  if (phi_shape_is<16, 8, 2>(a.t))  // n_phi = 512
-    return launch_nl_bouss_s<MAG, CHEM, SPLIT_IO, PhiShape<16, 8, 2>, 256>(a, st);
+  if (phi_shape_static(a.t)) switch (a.t.fft_b) {
+#define X(b) \
+  case b: return launch_nl_bouss_s<MAG, CHEM, SPLIT_IO, PhiShape<16, b, 2>, 256>(a, st);
+      MT_PHI_STATIC_B(X)
+#undef X
+      default: break;
+    }
   const int r = phi_max_radix(a.t);
   if (r <= 12) return launch_nl_bouss_s<MAG, CHEM, SPLIT_IO, PhiShapeRt<12>, 128>(a, st);
   if (r <= 18) return launch_nl_bouss_s<MAG, CHEM, SPLIT_IO, PhiShapeRt<18>, 256>(a, st);

@@ -480,11 +480,17 @@ __device__ __forceinline__ void phi_store_rows(const cplx<R>* buf, const SH& sh,
   }
 }
 
+// Shapes that the FP64 phi stages compile in: all of outer radix 16, n_phi 512, 640,
+// 768, 960, 1024 and 1152, the inner radices of MT_PHI_STATIC_B.  There strides and
+// divisions become constants and the radix switch goes, and with PhiShapeRt the
+// Boussinesq stages take 4 to 12 % longer, the anelastic ones 3 to 7 % (65 levels,
+// FP64 contractions: n_phi 512 1.91 and 2.08 ms, 768 5.53 and 5.76, 640 anelastic
+// 4.20 and 4.29).  Each shape costs twelve kernels; of the lengths without one, the
+// short ones have stages bound by their launches and Legendre contractions.
+#define MT_PHI_STATIC_B(X) X(8) X(10) X(12) X(15) X(16) X(18)
+inline bool phi_shape_static(const Tables& t) { return t.fft_a == 16 && t.fft_f == 2; }
+
 // Largest radix, slots of a row and table entries of the plan's shape (host).
-template <int A, int B, int F>
-inline bool phi_shape_is(const Tables& t) {
-  return t.fft_a == A && t.fft_b == B && t.fft_f == F;
-}
 inline int phi_max_radix(const Tables& t) { return t.fft_a > t.fft_b ? t.fft_a : t.fft_b; }
 inline int phi_row_len(const Tables& t) { return (t.fft_a * ((t.fft_f * t.fft_b) | 1)) | 1; }
 inline int phi_tw_len(const Tables& t) { return (2 * t.fft_a - 1) * t.fft_f * t.fft_b; }

@@ -81,7 +81,7 @@ def test_rows_of_every_length(n_phi, precision, tol):
         assert np.abs(back - ref).max() < tol * np.abs(ref).max(), (n_phi, cols)
 
 
-# n_phi 30 (F = 1), 300 (15 x 10), 500 (25 x 5), 1000 (25 x 10)
+# n_phi 30 (F = 1), 300 (15 x 5), 500 (25 x 5), 1000 (25 x 10)
 STAGES = [(40, 4, 5, True, True), (100, 1, 4, True, False), (166, 1, 3, True, False),
           (333, 1, 3, False, False)]
 PAIR = {"Advt": "Advp", "Advp": "Advt", "VxBt": "VxBp", "VxBp": "VxBt"}
@@ -123,3 +123,39 @@ def test_stages_at_other_row_lengths(l_max, minc, N, l_mag, l_chem, anel):
             err = np.abs(out[k].cpu().numpy() - ref[k]).max() / scale
             assert err < tol, (precision, k, err)
         assert np.abs(dt.cpu().numpy() - rdt).max() < max(tol, 1e-12) * np.abs(rdt).max()
+
+
+@pytest.mark.parametrize("anel", [False, True])
+def test_compiled_shapes(anel):
+    """The FP64 phi stages at every row length they compile in (512 to 1152, outer
+    radix 16) against the run-time shape of n_phi 600: the products are quadratic, so
+    at l_max 64 any n_phi above 192 gives the same spectra, to the stages' FP64 and
+    digit-split tolerances."""
+    from magic_b200 import Plan
+
+    l_max, N = 64, 5
+    rng = np.random.default_rng(16)
+    make = lambda n, prec: Plan(l_max, precision=prec, n_theta_max=100, n_phi_max=n)
+    q = make(600, "fp64")
+    names = ("w", "dw", "ddw", "z", "dz", "s", "b", "db", "ddb", "aj", "dj", "xi")
+    f = {}
+    for k in names:
+        x = rng.standard_normal((q.lm_max, N)) + 1j * rng.standard_normal((q.lm_max, N))
+        x *= ((q.lm2l + 1.0) ** -1.5)[:, None]
+        x[q.lm2m == 0] = x[q.lm2m == 0].real
+        f[k] = torch.from_numpy(x).cuda()
+    if anel:
+        prof, args = ostage.anel_profiles(N, l_max=l_max), (200.0, 0.3, 0.2, 2.5, 1.0, 0.2)
+    else:
+        prof, args = ostage.bouss_profiles(N, l_max=l_max), (200.0, 2.5, 1.0, 0.2)
+    prof = {k: torch.as_tensor(np.ascontiguousarray(v)).cuda() for k, v in prof.items()}
+    run = lambda p, **kw: (p.nl_anel if anel else p.nl_bouss)(f, prof, *args, **kw)[0]
+    for kw in (dict(l_mag=True, l_chem=False), dict(l_mag=False, l_chem=True)):
+        ref = run(q, **kw)
+        for n_phi in (512, 640, 768, 960, 1024, 1152):
+            for precision, tol in (("fp64", 1e-12), ("ozaki", 5e-13 * l_max ** 2)):
+                out = run(make(n_phi, precision), **kw)
+                for k in ref:
+                    scale = max(ref[j].abs().max().item() for j in (k, PAIR.get(k, k)))
+                    err = (out[k] - ref[k]).abs().max().item()
+                    assert err < tol * scale, (n_phi, precision, k, err / scale)
