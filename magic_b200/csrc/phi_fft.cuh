@@ -29,7 +29,7 @@
 // stride S nearly so the load and store phases (lanes on consecutive fields of
 // one k); the outer step reads runs of consecutive slots.
 //
-// Radices (2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16, 18, 20, 25, 27) cover every H with
+// Radices (2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16, 18, 25, 27) cover every H with
 // factors 2, 3, 5 up to 584 in the two steps; phi_factor (tables.cu) picks the
 // pair.
 #pragma once
@@ -285,7 +285,7 @@ __device__ __forceinline__ void phi_inner_r(cplx<T>* buf, int nrows, const SH& s
 }
 
 #define MT_PHI_RADICES(X) \
-  X(2) X(3) X(4) X(5) X(6) X(8) X(9) X(10) X(12) X(15) X(16) X(18) X(20) X(25) X(27)
+  X(2) X(3) X(4) X(5) X(6) X(8) X(9) X(10) X(12) X(15) X(16) X(18) X(25) X(27)
 
 template <bool INV, class SH, typename T>
 __device__ __forceinline__ void phi_outer(cplx<T>* buf, int nrows, const SH& sh,

@@ -154,7 +154,7 @@ __global__ void k_phi_tw1(int A, int B, int F, double2* tw) {
 // the inner step), then the smallest larger radix; false if H has a factor other
 // than 2, 3, 5.
 static bool phi_factor(int H, int* a, int* b, int* f) {
-  static const int radix[] = {1, 2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16, 18, 20, 25, 27};
+  static const int radix[] = {1, 2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16, 18, 25, 27};
   *f = H % 2 == 0 ? 2 : 1;
   const int n = H / *f;
   int best = 1 << 30;
