@@ -10,7 +10,8 @@
 // vector components), written as north/south Fourier rows for the analysis
 // packing kernel.  One CTA = (theta row, up to kPhiRows rows); the FFT is the
 // half-warp one (fft_hw.cuh) for n_phi = 256, 384, 512, 768, Stockham passes
-// (fft.cuh) for 250 and 500, and the two-step one (phi_fft.cuh) otherwise.
+// (fft.cuh) where the two steps would be too few transforms of 25 or 27 points
+// (launch_split_phi), and the two-step one (phi_fft.cuh) otherwise.
 #include "fft_hw.cuh"
 #include "phi_fft.cuh"
 #include "split_kernels.cuh"
@@ -216,13 +217,10 @@ __global__ void __launch_bounds__(kPhiThreads, SH::kMax <= 12 ? 4 : 3)
   }
 }
 
-// Rows of 125 = 25 x 5 points (n_phi 250 and 500): block-wide Stockham passes of
-// radices up to 8 (fft.cuh, kStRows rows at a time through a scratch buffer).  A row
-// has no more than ten 25-point transforms, each a long chain for one thread, and
-// three passes of radix 5 are as short as two steps.  A round of the four transforms
-// at n_phi 250, l_max 327, 7 columns: 333 us in two steps, 301 in passes; at n_phi
-// 500, l_max 163, 14 columns: 285 and 276; but at n_phi 800, l_max 266, 30 columns (20
-// x 10) 740 and 819, at n_phi 1000 (25 x 10), l_max 333, 1190 and 1328.
+// Few transforms of 25 or 27 points: block-wide Stockham passes of radices up to 8
+// (fft.cuh, kStRows rows at a time through a scratch buffer).  Such a transform is a
+// long chain for one thread, and a step of few leaves most threads idle; passes of
+// radix 5 and 3 share the work among more.
 constexpr int kStRows = 7;
 
 __global__ void __launch_bounds__(kPhiThreads) k_split_to_grid_st(SplitPhiArgs a) {
@@ -351,9 +349,18 @@ int launch_split_phi(bool to_grid, const SplitPhiArgs& a, cudaStream_t st) {
     case 768: return launch_hw<24>(to_grid, a, st);
     default: break;
   }
-  if (a.t.fft_a > 18 && a.t.fft_b <= 5) return launch_st(to_grid, a, st);
-  return phi_max_radix(a.t) <= 12 ? launch_rows<PhiShapeRt<12>>(to_grid, a, st)
-                                  : launch_rows<PhiShapeRt<27>>(to_grid, a, st);
+  const int r = phi_max_radix(a.t);
+  // Radix 25 or 27 (n_phi 250, 486, 500, 750, 800, 810, 972, 1000).  On at most eight
+  // rows passes take scal_to_spat from 138 to 128 us (n_phi 1000, 1 column), from 86 to 77
+  // (750), from 95 to 88 (486, l_max 324, minc 2, 8 columns); with more rows a round of
+  // the four transforms takes 740 us in two steps and 819 in passes (n_phi 800, l_max
+  // 266, 30 columns), 1190 and 1328 (1000, l_max 333).  With an inner step of five
+  // points (250 and 500) a row is at most ten 25-point transforms, and three passes are as
+  // short as two steps at any number: 301 us in passes and 333 in steps (250, l_max
+  // 327, 7 columns), 276 and 285 (500, l_max 163, 14).
+  if (r > 18 && (a.nrows <= 8 || a.t.fft_b <= 5)) return launch_st(to_grid, a, st);
+  return r <= 12 ? launch_rows<PhiShapeRt<12>>(to_grid, a, st)
+                 : launch_rows<PhiShapeRt<27>>(to_grid, a, st);
 }
 
 }  // namespace mt
