@@ -151,13 +151,15 @@ __global__ void __launch_bounds__(kPackThreads, 4) k_syn_pack(SplitSynArgs a) {
     cp_async_commit();
     // while these arrive, the rows of the block a wave later (four an SM) are asked
     // into L2: stage at l_max 85 on 49 levels 257 -> 253 us, at l_max 127 on 65 levels
-    // 609 -> 604
-    constexpr int kAhead = 4 * 148;
-    const int64_t id = ((int64_t)mc * gridDim.y + c) * gridDim.x + rt + kAhead;
-    const int rt2 = (int)(id % gridDim.x), c2 = (int)(id / gridDim.x % gridDim.y);
-    const int64_t mc2 = id / gridDim.x / gridDim.y;
-    if (mc2 < gridDim.z) {
-      const int nlm2 = t.l_max - (int)mc2 * t.minc + 1, l2 = rt2 * kSplitRows / a.row_per_level;
+    // 609 -> 604.  The id's divisions are 32-bit ones, and only where that block exists:
+    // 64-bit ones in every block cost a small call 1 to 2 us (scal_to_spat at n_phi 250,
+    // minc 2, 2 columns 44 -> 46).
+    const unsigned id = (mc * gridDim.y + c) * gridDim.x + rt + 4 * kSms;
+    if (id < gridDim.x * gridDim.y * gridDim.z) {
+      const unsigned row_id = id / gridDim.x;
+      const int mc2 = row_id / gridDim.y, c2 = row_id - mc2 * gridDim.y;
+      const int rt2 = id - row_id * gridDim.x;
+      const int nlm2 = t.l_max - mc2 * t.minc + 1, l2 = rt2 * kSplitRows / a.row_per_level;
       const int nb = min(a.stg_lev, a.n_lev - l2) * 16;
       const int64_t off0 = (int64_t)(t.lstart[mc2] + 32 * c2) * a.ld + l2;
       for (int e = tid; e < 32 * a.narr; e += kPackThreads) {
