@@ -17,12 +17,17 @@ constexpr int kColsPerCta = 8;  // real columns (grid rows) per CTA
 // radices on at most kFewCols columns, where a step has too few transforms for
 // 256 threads (n_phi 250, 3 columns: 75 and 15) and the registers of a radix-25
 // transform allow two CTAs of that size only: a round trip of 3 columns at l_max
-// 327, minc 4 takes 173 us with 256 threads, 165 with 128.
-constexpr int kFftThreads = 256, kFewThreads = 128, kFewCols = 4;
+// 327, minc 4 takes 173 us with 256 threads, 165 with 128.  Up to two CTAs an SM
+// (kFewRows theta rows) those get all the registers they ask for instead of a
+// quarter of the SM's, and the radix-25 and 27 transforms don't spill: 1 column at
+// n_phi 500, l_max 166, analysis 20.9 -> 18.9 us, synthesis 20.0 -> 18.0; above, the
+// limit is the better (n_phi 750, l_max 250: 26 against 29 us).
+constexpr int kFftThreads = 256, kFewThreads = 128, kFewCols = 4, kFewRows = 2 * kSms;
 
-template <class SH, int T>
-__global__ void __launch_bounds__(T, T == kFewThreads ? 4 : SH::kMax <= 12 ? 3 : 2)
-    k_fourier_to_grid(ToGridArgs a) {
+constexpr int fft_ctas(int kMax) { return kMax <= 12 ? 3 : 2; }
+
+template <class SH, int T, int kCtas>
+__global__ void __launch_bounds__(T, kCtas) k_fourier_to_grid(ToGridArgs a) {
   extern __shared__ double smem[];
   cplx<double>* buf = reinterpret_cast<cplx<double>*>(smem);
   const Tables& t = a.t;
@@ -98,9 +103,8 @@ __global__ void __launch_bounds__(T, T == kFewThreads ? 4 : SH::kMax <= 12 ? 3 :
   }
 }
 
-template <class SH, int T>
-__global__ void __launch_bounds__(T, T == kFewThreads ? 4 : SH::kMax <= 12 ? 3 : 2)
-    k_grid_to_fourier(ToFourierArgs a) {
+template <class SH, int T, int kCtas>
+__global__ void __launch_bounds__(T, kCtas) k_grid_to_fourier(ToFourierArgs a) {
   extern __shared__ double smem[];
   cplx<double>* buf = reinterpret_cast<cplx<double>*>(smem);
   const Tables& t = a.t;
@@ -150,10 +154,10 @@ static size_t fft_smem(const Tables& t) {
   return ((size_t)kColsPerCta * phi_row_len(t) + phi_tw_len(t)) * sizeof(double2);
 }
 
-template <int kMax, int T = kFftThreads>
+template <int kMax, int T = kFftThreads, int kCtas = fft_ctas(kMax)>
 static int launch_to_grid(const ToGridArgs& a, cudaStream_t st) {
   const size_t sm = fft_smem(a.t);
-  auto kern = k_fourier_to_grid<PhiShapeRt<kMax>, T>;
+  auto kern = k_fourier_to_grid<PhiShapeRt<kMax>, T, kCtas>;
   MT_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   dim3 grid((a.ncols + kColsPerCta - 1) / kColsPerCta, a.t.n_theta);
   kern<<<grid, T, sm, st>>>(a);
@@ -161,10 +165,10 @@ static int launch_to_grid(const ToGridArgs& a, cudaStream_t st) {
   return MT_OK;
 }
 
-template <int kMax, int T = kFftThreads>
+template <int kMax, int T = kFftThreads, int kCtas = fft_ctas(kMax)>
 static int launch_to_fourier(const ToFourierArgs& a, cudaStream_t st) {
   const size_t sm = fft_smem(a.t);
-  auto kern = k_grid_to_fourier<PhiShapeRt<kMax>, T>;
+  auto kern = k_grid_to_fourier<PhiShapeRt<kMax>, T, kCtas>;
   MT_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   dim3 grid((a.ncols + kColsPerCta - 1) / kColsPerCta, a.t.n_theta);
   kern<<<grid, T, sm, st>>>(a);
@@ -176,15 +180,18 @@ int launch_fourier_to_grid(const ToGridArgs& a, cudaStream_t st) {
   const int r = phi_max_radix(a.t);
   if (r <= 12) return launch_to_grid<12>(a, st);
   if (r <= 18) return launch_to_grid<18>(a, st);
-  return a.ncols <= kFewCols ? launch_to_grid<27, kFewThreads>(a, st) : launch_to_grid<27>(a, st);
+  if (a.ncols > kFewCols) return launch_to_grid<27>(a, st);
+  return a.t.n_theta <= kFewRows ? launch_to_grid<27, kFewThreads, 2>(a, st)
+                                 : launch_to_grid<27, kFewThreads, 4>(a, st);
 }
 
 int launch_grid_to_fourier(const ToFourierArgs& a, cudaStream_t st) {
   const int r = phi_max_radix(a.t);
   if (r <= 12) return launch_to_fourier<12>(a, st);
   if (r <= 18) return launch_to_fourier<18>(a, st);
-  return a.ncols <= kFewCols ? launch_to_fourier<27, kFewThreads>(a, st)
-                             : launch_to_fourier<27>(a, st);
+  if (a.ncols > kFewCols) return launch_to_fourier<27>(a, st);
+  return a.t.n_theta <= kFewRows ? launch_to_fourier<27, kFewThreads, 2>(a, st)
+                                 : launch_to_fourier<27, kFewThreads, 4>(a, st);
 }
 
 // Largest n_phi that the row FFTs' two radices cover (phi_fft.cuh).
