@@ -252,7 +252,8 @@ def stream_handle(device):
 
 # torch carries out a conjugation or a sign lazily: x.conj() is a view of x's memory
 # with a bit set, and .to() and .contiguous() may hand the same memory back.  Kernels
-# read and write the memory.
+# read and write the memory.  (.conj() sets its bit on complex tensors; the negation
+# bit comes with the imaginary part of one of those.)
 
 def plain(x):
     """x as a kernel may read it: its memory holds its values."""

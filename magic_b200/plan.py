@@ -178,7 +178,8 @@ class Plan:
             raise ValueError(f"{name}: expected shape (lm_max={self.lm_max},[B])")
         if x.dtype != _CD:
             x = x.to(_CD)
-        x = plain(x)
+        if x.is_conj():
+            x = x.resolve_conj()
         if n == 1:
             if x.stride(0) < 1:
                 x = x.contiguous()
@@ -196,7 +197,9 @@ class Plan:
             raise ValueError(f"{name}: expected shape ([B,] {self.n_theta_max}, {self.n_phi_max})")
         if x.dtype != _RD:
             x = x.to(_RD)
-        return plain(x).contiguous(), x.size(0) if n == 3 else 1, n == 2
+        if x.is_neg():
+            x = x.resolve_neg()
+        return x.contiguous(), x.size(0) if n == 3 else 1, n == 2
 
     def _new_grid(self, B, one):
         shape = (self.n_theta_max, self.n_phi_max)
