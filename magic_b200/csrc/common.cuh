@@ -38,7 +38,7 @@ void set_error(const std::string& msg);
 
 constexpr int kMaxFftStages = 24;
 
-// SMs of a B200, as a measure of waves (persistent grids ask the device).
+// SMs of a B200, as a measure of waves and look-aheads (persistent grids ask the device).
 constexpr int kSms = 148;
 
 // Device-side view of the horizontal tables, passed by value to kernels.

@@ -690,7 +690,7 @@ int launch_synth_split(const SplitSynArgs& a, cudaStream_t st) {
   const size_t sm = L.total();
   MT_CHECK_CUDA(cudaFuncSetAttribute(k_synth_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)sm));
-  int dev = 0, nsm = 148;
+  int dev = 0, nsm = kSms;
   MT_CHECK_CUDA(cudaGetDevice(&dev));
   MT_CHECK_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   const int nitems = ntiles * 2 * a.s.nthtile * a.t.n_m;

@@ -23,8 +23,8 @@ struct BoussFields {
 
 // One CTA per (theta row, level).  Block-wide phases: load with the real-row
 // pre-processing, inverse row FFTs (phi_fft.cuh), products, forward row FFTs,
-// store; two CTAs of T threads share an SM, so one's loads overlap the
-// other's arithmetic.
+// store; two CTAs of 256 threads or four of 128 share an SM (where their rows fit
+// its shared memory), so one's loads overlap another's arithmetic.
 template <bool MAG, bool CHEM, bool SPLIT_IO, class SH, int T>
 __global__ void __launch_bounds__(T, 512 / T) k_nl_bouss(NlBoussArgs a) {
   using BF = BoussFields<MAG, CHEM>;

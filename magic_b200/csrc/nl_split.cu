@@ -227,7 +227,7 @@ __global__ void __maxnreg__(72)
   // at 9 % of its bandwidth.  Stage at l_max 85 on 49 levels 257 -> 254 us, at l_max
   // 127 on 65 levels 609 -> 599.
   if ((row & 1) == 0) {
-    constexpr int kAhead = 4 * 148;
+    constexpr int kAhead = 4 * kSms;
     const int id = r * gridDim.x + row + kAhead, r2 = id / gridDim.x, row2 = id - r2 * gridDim.x;
     if (r2 < a.n_r) {
       const float* x = a.Fs + (int64_t)(row2 >> 1) * a.fs_j + (int64_t)r2 * 2 * NFI;

@@ -112,7 +112,7 @@ __global__ void k_get_nl_anel(GridNlArgs a) {
 
 int launch_get_nl_grid(bool anel, const GridNlArgs& a, cudaStream_t st) {
   int64_t total = (int64_t)a.n_r * a.nt * a.np;
-  int blocks = (int)std::min<int64_t>((total + 255) / 256, 148 * 16);
+  int blocks = (int)std::min<int64_t>((total + 255) / 256, kSms * 16);
   if (blocks < 1) blocks = 1;
   if (anel) k_get_nl_anel<<<blocks, 256, 0, st>>>(a);
   else k_get_nl<<<blocks, 256, 0, st>>>(a);

@@ -883,7 +883,7 @@ int launch_oz_synth(const OzSynArgs& a, cudaStream_t st) {
   // a sum has one term per degree: P on one parity of l - m, dP on the other
   auto gemm = a.t.l_max + 1 <= kOzPairTerms ? k_oz_synth_gemm<true> : k_oz_synth_gemm<false>;
   MT_CHECK_CUDA(cudaFuncSetAttribute(gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  int dev = 0, nsm = 148;
+  int dev = 0, nsm = kSms;
   MT_CHECK_CUDA(cudaGetDevice(&dev));
   MT_CHECK_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   const int nitems = ntiles * a.z.nthtile * a.t.n_m;
@@ -928,7 +928,7 @@ inline size_t oz_ana_pack_smem(int nhs, int rb) {
 // -> 5.43 ms, anelastic at l_max 383 on 129 levels 15.0 -> 14.83, at l_max 127 on 65
 // levels 1.033 -> 0.998 ms with the third CTA that 80 registers allow where shared
 // memory does.
-constexpr int kOzPackAhead = 2 * 148;
+constexpr int kOzPackAhead = 2 * kSms;
 
 template <int RB>
 __global__ void __launch_bounds__(kOzPackThreads, 3) k_oz_ana_pack(OzAnaArgs a) {
@@ -1291,7 +1291,7 @@ int launch_oz_anal(const OzAnaArgs& a, cudaStream_t st) {
   // a sum has one term per theta pair
   auto gemm = a.t.nhs <= kOzPairTerms ? k_oz_anal_gemm<true> : k_oz_anal_gemm<false>;
   MT_CHECK_CUDA(cudaFuncSetAttribute(gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  int dev = 0, nsm = 148;
+  int dev = 0, nsm = kSms;
   MT_CHECK_CUDA(cudaGetDevice(&dev));
   MT_CHECK_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   const int nitems = ntiles * 2 * a.z.nlt * a.t.n_m;

@@ -361,13 +361,15 @@ __device__ __forceinline__ void phi_twiddles_to_smem(cplx<T>* tws, const SH& sh,
 
 // The phases of a fused stage around the row FFTs (T = blockDim.x threads).
 
-// Asks the L2 for the rows that the CTA about to follow this one on its SM will
-// load: kAhead = 2 CTAs x 148 SMs further along the grid (x fastest).  at(row, r)
-// is the address of its k = 0 entry, `pitch` doubles from one k to the next; two
-// lines cover the NF <= 19 complex values of one k.
+// Asks the L2 for the rows of a CTA one wave further along the grid (x fastest), so
+// that they are there when it takes this one's place: a wave is 512 threads an SM,
+// what the stages' launch bounds ask for (where shared memory holds fewer CTAs, the
+// rows wait in the L2 for longer).  at(row, r) is the address of its k = 0 entry,
+// `pitch` doubles from one k to the next; the first and the last line of the NF
+// complex values of one k are asked for.
 template <int NF, int T, typename At>
 __device__ __forceinline__ void phi_prefetch(int M, int64_t pitch, At at) {
-  constexpr int kAhead = 2 * 148;
+  constexpr int kAhead = 512 / T * kSms;
   const int id = blockIdx.y * gridDim.x + blockIdx.x + kAhead;
   const int row = id / gridDim.x, r = id - row * gridDim.x;
   if (row >= (int)gridDim.y) return;

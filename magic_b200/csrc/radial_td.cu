@@ -356,7 +356,7 @@ static int radial_apply_n(const mt_radial_op* const* ops, int nop, int nrows, co
   const size_t sm = wpb * per_warp;
   MT_CHECK_CUDA(cudaFuncSetAttribute(k_radial_apply, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)sm));
-  int dev = 0, nsm = 148;
+  int dev = 0, nsm = kSms;
   MT_CHECK_CUDA(cudaGetDevice(&dev));
   MT_CHECK_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   const int blocks = (int)std::min<int64_t>((nrows + wpb - 1) / wpb, (int64_t)nsm * 16);
