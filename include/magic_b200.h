@@ -271,12 +271,6 @@ MT_API int mt_nl_anel_f64(const mt_plan* plan, int n_r, const mt_anel_in* in,
                const mt_anel_out* out, const mt_anel_stage_params* p, double* dtrkc,
                double* dthkc, void* work, size_t work_bytes, void* stream);
 
-/* Self-test of the device-side failure detection (no reference counterpart):
- * one CTA waits on an mbarrier that nothing completes, gives up after
- * `spins` polls, writes 99 to the device int *status (which the caller zeroes
- * first) and returns, so the context stays usable.  The tensor-core kernels
- * use the same bounded wait (2^22 polls) and report their own codes in the
- * first int of their workspace. */
 /* ---- radial operators ---------------------------------------------------
  * A real n_r x n_r matrix D applied along the radial axis of complex rows:
  * out[b][j] = sum_k D[j][k] in[b][k] for b < nrows, rows of n_r complex
@@ -517,7 +511,21 @@ MT_API size_t mt_energy_workspace(const mt_plan* plan);
 MT_API int mt_energy(const mt_plan* plan, int n_r, const mt_energy_args* e, double* out,
                      void* work, size_t work_bytes, void* stream);
 
+/* Self-test of the device-side failure detection (no reference counterpart):
+ * one CTA waits on an mbarrier that nothing completes, gives up after
+ * `spins` polls, writes 99 to the device int *status (which the caller zeroes
+ * first) and returns, so the context stays usable.  The tensor-core kernels
+ * use the same bounded wait (2^22 polls) and report their own codes in the
+ * first int of their workspace. */
 MT_API int mt_selftest_wait_timeout(int* status, long long spins, void* stream);
+
+/* Self-test of the digit-split epilogues' two sums of an accumulator column's six
+ * weight groups (no reference counterpart): for n columns of six int32 group words
+ * (device, column by column) the sum 2^35 sum_g 2^(-7 g) C_g as the kernels form it
+ * through int32 pairs and as they form it in FP64 (device, n each).  *pair_terms
+ * (host) is the largest number of terms a sum may have for the first form. */
+MT_API int mt_selftest_oz_combine(const int* groups, int n, double* paired, double* plain,
+                                  int* pair_terms, void* stream);
 
 /* ---- cross-run batching ------------------------------------------------- */
 

@@ -200,6 +200,7 @@ _PROTOS = {
     "mt_update_wp": (C.c_int, [C.c_void_p, C.c_int, C.POINTER(WpUpdate), C.c_void_p,
                                C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, _dp]),
     "mt_selftest_wait_timeout": (C.c_int, [_dp, C.c_longlong, _dp]),
+    "mt_selftest_oz_combine": (C.c_int, [_dp, C.c_int, _dp, _dp, C.POINTER(C.c_int), _dp]),
     "mt_copy_levels": (C.c_int, [C.c_int, _dp, C.c_int, _dp]),
     "mt_device_status": (C.c_int, [_dp, C.POINTER(C.c_int), _dp]),
     "mt_noalloc_status": (C.c_int, [C.POINTER(C.c_int), _dp]),

@@ -1748,6 +1748,12 @@ int mt_selftest_wait_timeout(int* status, long long spins, void* stream) {
   return launch_selftest_wait(status, (long)spins, (cudaStream_t)stream);
 }
 
+int mt_selftest_oz_combine(const int* groups, int n, double* paired, double* plain,
+                           int* pair_terms, void* stream) {
+  MT_REQUIRE(groups && n > 0 && paired && plain && pair_terms, MT_ERR_ARG, "bad argument");
+  return launch_selftest_oz_combine(groups, n, paired, plain, pair_terms, (cudaStream_t)stream);
+}
+
 int mt_device_status(const void* work, int* code, void* stream) {
   MT_REQUIRE(work && code, MT_ERR_ARG, "work and code pointers required");
   cudaStream_t st = (cudaStream_t)stream;

@@ -1300,4 +1300,24 @@ int launch_oz_anal(const OzAnaArgs& a, cudaStream_t st) {
   return MT_OK;
 }
 
+// Both sums of the epilogues on given group words.
+__global__ void k_selftest_oz_combine(const int* groups, int n, double* paired, double* plain) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  uint32_t c[kOzGroups][1], q[3][1];
+#pragma unroll
+  for (int g = 0; g < kOzGroups; ++g) c[g][0] = (uint32_t)groups[(int64_t)i * kOzGroups + g];
+  oz_pair_groups(c, q);
+  paired[i] = oz_combine_q(q, 0);
+  plain[i] = oz_combine_u(c, 0);
+}
+
+int launch_selftest_oz_combine(const int* groups, int n, double* paired, double* plain,
+                               int* pair_terms, cudaStream_t st) {
+  *pair_terms = kOzPairTerms;
+  k_selftest_oz_combine<<<(n + 127) / 128, 128, 0, st>>>(groups, n, paired, plain);
+  MT_CHECK_CUDA(cudaGetLastError());
+  return MT_OK;
+}
+
 }  // namespace mt

@@ -112,5 +112,7 @@ size_t oz_syn_image_bytes(int nrows, int64_t total_chunks);
 size_t oz_ana_image_bytes(int n_m, int nhs, int n_lev, int lev_tile);
 int launch_oz_synth(const OzSynArgs& a, cudaStream_t st);
 int launch_oz_anal(const OzAnaArgs& a, cudaStream_t st);
+int launch_selftest_oz_combine(const int* groups, int n, double* paired, double* plain,
+                               int* pair_terms, cudaStream_t st);
 
 }  // namespace mt
