@@ -1,6 +1,8 @@
 // Shared-memory FFTs of the phi stage: complex arithmetic, register DFTs, and the
 // block-wide Stockham chain of the FP32 Boussinesq stage at row lengths without
-// a half-warp form (the other kernels use phi_fft.cuh and fft_hw.cuh).
+// a half-warp form and of the split transforms that are too few 25- and 27-point
+// DFTs for two steps (split_transforms.cu); the other kernels use phi_fft.cuh and
+// fft_hw.cuh.
 //
 // Each real field row of length N = n_phi is transformed on its own through a
 // complex FFT of half length H = N/2 (z_n = x_2n + i x_2n+1), so rounding of

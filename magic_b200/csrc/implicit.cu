@@ -626,10 +626,11 @@ __device__ __forceinline__ void solve_rows_to(const double* __restrict__ Ml, int
 
 // kBand: banded factors.  The solve is one warp's serial chain while the others
 // wait, so what counts is how many CTAs an SM holds, and compiled apart from the
-// tensor-pipe tile the registers allow more of them: four here (five spill) and
-// three in k_update_poloidal, against three and two in one kernel with the dense
-// solve.  All updates of a step at l_max 255 on 97 finite-difference levels: 1061
-// -> 950 us (five CTAs here: 1244; two in k_update_poloidal: 962).
+// tensor-pipe tile the registers allow more of them: four here (64 registers, 56
+// bytes spilled) and three in k_update_poloidal (80, 392 bytes), against three and
+// two in one kernel with the dense solve.  All updates of a step at l_max 255 on 97
+// finite-difference levels: 1061 -> 950 us (five CTAs here, with more spilled: 1244;
+// two in k_update_poloidal, with nothing spilled: 962).
 // Otherwise a dense solve with kNt n-tiles per warp.
 template <bool kStaged, int kNt, bool kBand>
 __global__ void __launch_bounds__(Bounds<kStaged, 2>::kThreads,

@@ -1,4 +1,5 @@
-// The FP64 phi stage of the digit-split anelastic radial loop.
+// The FP64 phi stage of the anelastic radial loop, on the rows of the FP64 and of the
+// digit-split contractions.
 #include <algorithm>
 
 #include "nl_point.cuh"
@@ -8,14 +9,13 @@
 
 namespace mt {
 
-// The phi stage of the digit-split anelastic radial loop.  One CTA (256
-// threads) per (theta row, level): the synthesis wrote this hemisphere's
-// Fourier rows of the grid fields in FP64 (NlAnelArgs::Fs64; field order of
-// nl_point.cuh), the kernel inverse-transforms them in place (phi_fft.cuh),
-// evaluates get_nl_anel (magic_torch/get_nl_anel.py:63-136, viscous and Ohmic
-// heating included) and the Courant maxima (magic_torch/courant.py:25-77) at
-// every grid point in FP64, and forward-transforms the 10-13 products into the
-// weighted rows the analysis reads (NlAnelArgs::G64).  Shared memory holds
+// One CTA (256 threads) per (theta row, level): the synthesis wrote this
+// hemisphere's Fourier rows of the grid fields in FP64 (NlAnelArgs::Fs64; field
+// order of nl_point.cuh), the kernel inverse-transforms them in place
+// (phi_fft.cuh), evaluates get_nl_anel (magic_torch/get_nl_anel.py:63-136, viscous
+// and Ohmic heating included) and the Courant maxima (magic_torch/courant.py:25-77)
+// at every grid point in FP64, and forward-transforms the 7 to 13 products into
+// the weighted rows the analysis reads (NlAnelArgs::G64).  Shared memory holds
 // only the rows (the twiddle tables are read through L1), so that two CTAs
 // share an SM without magnetic field at n_phi = 1152.  Velocity, its
 // derivatives and cvr are zero on the two boundary levels (radial_loop_anel

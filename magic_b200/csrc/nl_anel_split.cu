@@ -3,7 +3,7 @@
 // One CTA per (theta row, level), as k_nl_bouss_split_hw: the synthesis
 // delivers equatorially symmetric/antisymmetric Fourier rows of the 18 (19
 // with composition) grid fields, this kernel forms the hemisphere's rows,
-// transforms them (half-warp FFT for n_phi = 256, 384, 512, 768, block FFT
+// transforms them (half-warp FFT for n_phi = 256, 384, 512, 768, two-step row FFTs
 // otherwise), evaluates get_nl_anel (magic_torch/get_nl_anel.py:41-136,
 // viscous and Ohmic heating included) and the Courant maxima at every grid
 // point, and writes the weighted Fourier rows of the 10-13 products for the

@@ -159,3 +159,11 @@ def test_compiled_shapes(anel):
                     scale = max(ref[j].abs().max().item() for j in (k, PAIR.get(k, k)))
                     err = (out[k] - ref[k]).abs().max().item()
                     assert err < tol * scale, (n_phi, precision, k, err / scale)
+
+
+def test_longer_rows_are_refused():
+    """1200 is the first length of factors 2, 3, 5 above the limit, which the error names."""
+    from magic_b200 import MagicError, Plan
+
+    with pytest.raises(MagicError, match=r"limit \(1168\)"):
+        Plan(16, n_theta_max=24, n_phi_max=1200)
