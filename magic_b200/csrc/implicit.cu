@@ -625,16 +625,14 @@ __device__ __forceinline__ void solve_rows_to(const double* __restrict__ Ml, int
 }
 
 // kBand: banded factors.  The solve is one warp's serial chain while the others
-// wait, so what counts is how many CTAs an SM holds, and compiled apart from the
-// tensor-pipe tile the registers allow more of them: four here (64 registers, 56
-// bytes spilled) and three in k_update_poloidal (80, 392 bytes), against three and
-// two in one kernel with the dense solve.  All updates of a step at l_max 255 on 97
-// finite-difference levels: 1061 -> 950 us (five CTAs here, with more spilled: 1244;
-// two in k_update_poloidal, with nothing spilled: 962).
-// Otherwise a dense solve with kNt n-tiles per warp.
-template <bool kStaged, int kNt, bool kBand>
-__global__ void __launch_bounds__(Bounds<kStaged, 2>::kThreads,
-                                  Bounds<kStaged, kBand ? 4 : kNt == 2 ? 3 : 2>::kBlocks)
+// wait, so what counts is how many CTAs an SM holds (kCtas of 256 threads by its
+// registers), against what they spill for it; compiled apart from the tensor-pipe
+// tile the registers allow more of them.  Three here (80 registers) or four (64, 56
+// bytes spilled), two in k_update_poloidal (128) or three (80, 392 bytes), by
+// band_more_ctas.  Otherwise a dense solve with kNt n-tiles per warp.
+template <bool kStaged, int kNt, bool kBand, int kCtas>
+__global__ void __launch_bounds__(Bounds<kStaged, kCtas>::kThreads,
+                                  Bounds<kStaged, kCtas>::kBlocks)
     k_update_field(UsArgs a) {
   extern __shared__ __align__(16) double2 usbuf[];
   __shared__ int lm_row[16];
@@ -766,11 +764,11 @@ __device__ __forceinline__ void dn_zero(double (&acc)[kNt][4][2]) {
     for (int t = 0; t < 4; ++t) acc[i][t][0] = acc[i][t][1] = 0.0;
 }
 
-// CTAs of 16 orders with work: the orders m <= l of every degree.
-int dn_ctas(int l_max, int minc) {
-  int n = 0;
-  for (int l = 0; l <= l_max; ++l) n += (l / minc + 4 * kRows) / (4 * kRows);
-  return n;
+// CTAs of `rows` orders with work, ceil((l / minc + 1) / rows) for each degree l:
+// minc degrees for each l / minc = q < Q, the rest for Q.
+int update_ctas(int l_max, int minc, int rows) {
+  const int Q = l_max / minc, a = Q / rows, b = Q % rows;
+  return minc * (rows * a * (a + 1) / 2 + b * (a + 1)) + (l_max - Q * minc + 1) * (a + 1);
 }
 
 // Which field updates with dense operators run as one chain.  Up to 144 levels two
@@ -913,9 +911,9 @@ struct PwArgs {
 // Double-curl poloidal update (magic_torch/update_w_doublecurl.py:393-483):
 // same tiling as k_update_field; the CTA holding (l, m) = (0, 0) also solves
 // the l = 0 pressure (update_wp.py:173-194).
-template <bool kStaged, int kNt, bool kBand>
-__global__ void __launch_bounds__(Bounds<kStaged, 2>::kThreads,
-                                  Bounds<kStaged, kBand ? 3 : 2>::kBlocks)
+template <bool kStaged, int kNt, bool kBand, int kCtas>
+__global__ void __launch_bounds__(Bounds<kStaged, kCtas>::kThreads,
+                                  Bounds<kStaged, kCtas>::kBlocks)
     k_update_poloidal(PwArgs a) {
   extern __shared__ __align__(16) double2 pwbuf[];
   __shared__ int lm_row[16];
@@ -1057,6 +1055,26 @@ TileLaunch tile_launch(int n_r, int ldm, int l_max, int n_m, int row_buffers,
   t.smem = (size_t)row_buffers * rows * t.fs * sizeof(double2) +
            (band_bytes ? band_bytes : t.staged ? (size_t)2 * kKc * ldm * sizeof(double) : 0);
   return t;
+}
+
+// Whether a banded update takes the form with more CTAs an SM: an SM's registers hold
+// `more` warps of it, `fewer` of the other.  Its spills cost a third, so it is taken
+// where it saves more than a quarter of the waves.  (A form whose CTAs fill the
+// registers to the last warp, with warps that don't divide among the four
+// schedulers, is half a CTA short of that.)  Forms with more and with fewer, us:
+//   fields, l_max 127: 65 levels 38 and 28, 97 levels 42 and 55; l_max 235, minc 2, 35
+//   levels 32 and 26; l_max 255, 129 levels 203 and 220;
+//   poloidal, l_max 127: 57 levels 65 and 41, 65 levels 52 and 63; l_max 235, minc 2, 113
+//   levels 192 and 167; l_max 255, 97 levels 283 and 297.
+// One kernel with the dense solve had taken 36, 72, 33, 318; 43, 68, 183 and 321.
+bool band_more_ctas(const TileLaunch& t, int l_max, int minc, int more, int fewer) {
+  const int warps = t.threads / 32, ctas = update_ctas(l_max, minc, t.groups * kRows);
+  const auto waves = [&](int room) {
+    const int by_smem = (int)(227 * 1024 / (t.smem + 1024)), by_regs = room / warps;
+    const double full = by_regs * warps == room && warps % 4 ? by_regs - 0.5 : by_regs;
+    return std::ceil(ctas / (kSms * std::min<double>(by_smem, full)));
+  };
+  return waves(more) <= 0.72 * waves(fewer);
 }
 
 // ---------------------------------------------------------------------------
@@ -1784,7 +1802,7 @@ int mt_update_field(const mt_plan* p, int n_r, const mt_field_update* u, const m
   a.D1 = radial_op_view(D1);
   a.D2 = radial_op_view(D2);
   if (!solve->abd && n_r <= kStagedMaxR && D1->dense && D2->dense &&
-      field_chain(n_r, dn_ctas(p->l_max, p->minc))) {
+      field_chain(n_r, update_ctas(p->l_max, p->minc, 4 * kRows))) {
     const int nt_n = (n_r + 7) / 8, tiles = (nt_n + kDnMaxTiles - 1) / kDnMaxTiles;
     a.fs = n_r + ((4 - n_r) & 7);  // conflict-free A fragments
     const size_t sm = (size_t)4 * kRows * a.fs * sizeof(double2) +
@@ -1804,10 +1822,13 @@ int mt_update_field(const mt_plan* p, int n_r, const mt_field_update* u, const m
              "tile shape does not cover n_r");
   a.groups = t.groups;
   a.fs = t.fs;
-  auto kern = solve->abd ? (t.staged ? k_update_field<true, 2, true> : k_update_field<false, 2, true>)
-              : !t.staged ? k_update_field<false, 2, false>
-              : t.nt == 2 ? k_update_field<true, 2, false>
-                          : k_update_field<true, 4, false>;
+  auto kern = k_update_field<false, 2, false, 1>;
+  if (solve->abd)
+    kern = !t.staged ? k_update_field<false, 2, true, 1>
+           : band_more_ctas(t, p->l_max, p->minc, 32, 24) ? k_update_field<true, 2, true, 4>
+                                                          : k_update_field<true, 2, true, 3>;
+  else if (t.staged)
+    kern = t.nt == 2 ? k_update_field<true, 2, false, 3> : k_update_field<true, 4, false, 2>;
   MT_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t.smem));
   kern<<<t.grid, t.threads, t.smem, (cudaStream_t)stream>>>(a);
   MT_CHECK_CUDA(cudaGetLastError());
@@ -1896,11 +1917,13 @@ int mt_update_poloidal(const mt_plan* p, int n_r, const mt_poloidal_update* u,
              "tile shape does not cover n_r");
   a.groups = t.groups;
   a.fs = t.fs;
-  auto kern =
-      solve->abd ? (t.staged ? k_update_poloidal<true, 2, true> : k_update_poloidal<false, 2, true>)
-      : !t.staged ? k_update_poloidal<false, 2, false>
-      : t.nt == 2 ? k_update_poloidal<true, 2, false>
-                  : k_update_poloidal<true, 4, false>;
+  auto kern = k_update_poloidal<false, 2, false, 1>;
+  if (solve->abd)
+    kern = !t.staged ? k_update_poloidal<false, 2, true, 1>
+           : band_more_ctas(t, p->l_max, p->minc, 24, 16) ? k_update_poloidal<true, 2, true, 3>
+                                                          : k_update_poloidal<true, 2, true, 2>;
+  else if (t.staged)
+    kern = t.nt == 2 ? k_update_poloidal<true, 2, false, 2> : k_update_poloidal<true, 4, false, 2>;
   MT_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t.smem));
   kern<<<t.grid, t.threads, t.smem, (cudaStream_t)stream>>>(a);
   MT_CHECK_CUDA(cudaGetLastError());
@@ -1961,7 +1984,8 @@ int mt_update_wp(const mt_plan* p, int n_r, const mt_wp_update* u, const mt_lop*
   a.D3 = radial_op_view(D3);
   a.P0 = radial_op_view(P0);
   const int nt_s = (2 * n_r + 7) / 8, tiles = (nt_s + kDnMaxTiles - 1) / kDnMaxTiles;
-  if (D1->dense && D2->dense && D3->dense && wp_chain(nt_s, dn_ctas(p->l_max, p->minc))) {
+  if (D1->dense && D2->dense && D3->dense &&
+      wp_chain(nt_s, update_ctas(p->l_max, p->minc, 4 * kRows))) {
     const int fs = 2 * n_r + ((4 - 2 * n_r) & 7);
     a.ldd = lop_ld(n_r);
     const int ring = kKc * std::max(a.ldm, 2 * a.ldd);

@@ -452,3 +452,10 @@ def test_update_wp_uneven_tiles_vs_oracle():
     warp and dense derivatives by FMAs.  Scale 10: the conditioning's (81 / 65)^4 and
     the D3 norm's (81 / 65)^6 are 2.4 and 3.7 times those at 65 levels."""
     test_update_wp_vs_oracle(64, 1, 81, 2, 1e1)
+
+
+def test_banded_fields_four_ctas_vs_oracle():
+    """l_max = 127 on 97 finite-difference levels: the banded field kernel with four
+    CTAs an SM (one wave of them, where three take two); at l_max = 255 it is three."""
+    test_update_scalar_two_steps_vs_oracle("FD", 127, 97)
+    test_update_magnetic_vs_oracle("FD", 127, 97)
