@@ -94,6 +94,7 @@ class Plan:
         with torch.cuda.device(self.device):
             check(L.mt_plan_create(C.byref(desc), C.byref(h)))
         self._h = h
+        self._sizes = {}
         info = _lib.PlanInfo()
         check(L.mt_plan_get_info(h, C.byref(info)))
         self.l_max = info.l_max
@@ -169,6 +170,16 @@ class Plan:
     def _work(self, nbytes):
         return torch.empty(max(int(nbytes), 16), dtype=torch.uint8, device=self.device)
 
+    def _scratch(self, B, nf):
+        """Workspace of a transform of nf fields of B columns (its size is the plan's)."""
+        size = self._sizes.get((B, nf))
+        if size is None:
+            if len(self._sizes) >= 256:
+                self._sizes.clear()
+            size = _lib.lib().mt_transform_workspace(self._h, B, nf)
+            self._sizes[B, nf] = size
+        return self._work(size)
+
     def _spec(self, x, name):
         """(tensor, columns, row stride, whether 1-D) of a spectral argument."""
         if not isinstance(x, torch.Tensor) or x.device != self.device:
@@ -225,7 +236,7 @@ class Plan:
         X, B, ld, one = self._spec(Slm, "Slm")
         out = self._new_grid(B, one)
         L = _lib.lib()
-        ws = self._work(L.mt_transform_workspace(self._h, B, 1))
+        ws = self._scratch(B, 1)
         check(L.mt_scal_to_spat(self._h, X.data_ptr(), ld, B, out.data_ptr(), ws.data_ptr(),
                                 ws.numel(), self._stream()))
         self._watch(ws, "scal_to_spat")
@@ -235,7 +246,7 @@ class Plan:
         g, B, one = self._grid(sc, "sc")
         out = self._new_spec(B, one)
         L = _lib.lib()
-        ws = self._work(L.mt_transform_workspace(self._h, B, 1))
+        ws = self._scratch(B, 1)
         check(L.mt_scal_to_SH(self._h, g.data_ptr(), B, out.data_ptr(), B, ws.data_ptr(),
                               ws.numel(), self._stream()))
         self._watch(ws, "scal_to_SH")
@@ -252,7 +263,7 @@ class Plan:
             ld = Q.stride(0)
         outs = tuple(self._new_grid(B, one) for _ in range(3))
         L = _lib.lib()
-        ws = self._work(L.mt_transform_workspace(self._h, B, 3))
+        ws = self._scratch(B, 3)
         check(L.mt_torpol_to_spat(self._h, Q.data_ptr(), S.data_ptr(), T.data_ptr(), ld, B,
                                   *[o.data_ptr() for o in outs], ws.data_ptr(), ws.numel(),
                                   self._stream()))
@@ -266,7 +277,7 @@ class Plan:
             raise ValueError("vt and vp must have the same shape")
         S, T = self._new_spec(B, one), self._new_spec(B, one)
         L = _lib.lib()
-        ws = self._work(L.mt_transform_workspace(self._h, B, 2))
+        ws = self._scratch(B, 2)
         check(L.mt_spat_to_sphertor(self._h, gt.data_ptr(), gp.data_ptr(), B, S.data_ptr(),
                                     T.data_ptr(), B, ws.data_ptr(), ws.numel(), self._stream()))
         self._watch(ws, "spat_to_sphertor")
@@ -276,7 +287,7 @@ class Plan:
         X, B, ld, one = self._spec(Slm, "Slm")
         gt, gp = self._new_grid(B, one), self._new_grid(B, one)
         L = _lib.lib()
-        ws = self._work(L.mt_transform_workspace(self._h, B, 2))
+        ws = self._scratch(B, 2)
         check(L.mt_scal_to_grad_spat(self._h, X.data_ptr(), ld, B, int(scale_dlh),
                                      gt.data_ptr(), gp.data_ptr(), ws.data_ptr(), ws.numel(),
                                      self._stream()))
